@@ -263,9 +263,9 @@ __device__ __forceinline__ float adj_near_cell(const StepArgs& a, const NearTabl
     const LaneDir d = lane_dir(lane);
     const uint32_t t = static_cast<uint32_t>(__ldg(nt.cells + k));
     const uint32_t mask = __ldg(nt.mask + k);
-    const int sl = d.act ? __ldg(nt.slot + lane * nt.n + k) : 0;
-    const float q = d.act ? __ldg(nt.q + lane * nt.n + k) : 1.f;
-    const float wadd = d.act ? __ldg(nt.add + lane * nt.n + k) : 0.f;
+    const int sl = d.act ? __ldg(nt.slot + k * kQ + lane) : 0;
+    const float q = d.act ? __ldg(nt.q + k * kQ + lane) : 1.f;
+    const float wadd = d.act ? __ldg(nt.add + k * kQ + lane) : 0.f;
     const bool link = d.act && ((mask >> lane) & 1u);
     // the slot's value (a boundary fill is evaluated from its source) and
     // where its cotangent goes
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, LINKS ? 3 : 2) k_adj_step(const Step
   const int np = a.np, np3 = np * np * np;
   const int* gm = a.slot_map + static_cast<long long>(b) * np3;
   for (int k = threadIdx.x; k < np3; k += kThreads) smap[k] = gm[k];
-  const bool moving = a.blk_moving[b] != 0;  // uniform over the CTA
+  const bool moving = (a.blk_info[b] & kBlkMoving) != 0;  // uniform over the CTA
   __syncthreads();
   pdl_wait();
   const float* src = static_cast<const float*>(a.src);
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, LINKS ? 3 : 2) k_adj_step(const Step
       f[i] = __ldg(src + (sm >= 0 ? i * qs + sm : opp(i) * qs + t));
       lam[i] = lamY[i * qs + t];  // the output's cotangent, turned into the input's below
     }
-    if (moving) {  // moving-wall markers: only blocks flagged in blk_moving
+    if (moving) {  // moving-wall markers: only blocks with kBlkMoving
 #pragma unroll
       for (int i = 0; i < kQ; ++i) {
         const int sm = smap[P - a.off_pad[i]];

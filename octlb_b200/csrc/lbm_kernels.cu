@@ -21,7 +21,7 @@
 #include <string>
 #include <type_traits>
 
-#include "lbm_device.cuh"
+#include "lbm_step.cuh"
 
 namespace octlb_gpu {
 
@@ -59,34 +59,6 @@ __device__ __forceinline__ void source_slots(const StepArgs& a, const Cell& c, l
                              static_cast<int>(c.z) + 1 - cz(i));
     }
   }
-}
-
-// The 19 populations of cell t copied unchanged; all loads are issued
-// before the first store (for all the compiler knows, a store to row i may
-// alias the load from row i + 1, which would cost a round trip each).
-template <typename T>
-__device__ __forceinline__ void copy_cell(const T* src, T* dst, long long qs, uint32_t t) {
-  T v[kQ];
-#pragma unroll
-  for (int i = 0; i < kQ; ++i) v[i] = src[i * qs + t];
-#pragma unroll
-  for (int i = 0; i < kQ; ++i) dst[i * qs + t] = v[i];
-}
-
-// Torus-streamed halo population of an open block (block_lattice.h:70-89),
-// item k: copied without collision.
-template <typename T>
-__device__ __forceinline__ void rotate_item(const StepArgs& a, uint32_t k) {
-  if (k >= static_cast<uint32_t>(a.n_open)) return;
-  long long d, sl;
-  int i;
-  rotate_slots(a, k, d, sl, i);
-  const T* src = static_cast<const T*>(a.src);
-  T* dst = static_cast<T*>(a.dst);
-  if (sl >= a.halo_base && a.fill_of && a.fill_of[(sl - a.halo_base) * kQ + i] >= 0)
-    Store<T>::st(dst + i * a.qs + d, pull_value(a, src, i, sl), a.scale);  // source is a boundary fill
-  else
-    dst[i * a.qs + d] = src[i * a.qs + sl];
 }
 
 // ConstRhoBGK statistics of a step launch: this CTA's sum into
@@ -206,49 +178,6 @@ __global__ void __launch_bounds__(kThreads) k_step_cr(const StepArgs a) {
   rotate_item<T>(a, t - core_end);
 }
 
-// Cells flagged kFlagNear (links stream rule): the per-cell link rule of
-// block_lattice.cpp:613-672 with every table lookup done on the host --
-// direction i reads population i at nt.slot[i] and, where the rule applies,
-// reflects own[opp(i)] (half-way bounce-back, reflect-on-pull at the block
-// edge) or interpolates with Bouzidi (bouzidi_pull.h:8-26), then adds the
-// moving-wall term.  Then the same save / collide / store as k_step.  One
-// warp per cell, lane i on direction i; the collision gathers the 19 values
-// so every lane computes the moments exactly as bgk() does.
-template <typename T, int CM = kCollBgk>
-__device__ __forceinline__ float near_cell(const StepArgs& a, const NearTables& nt, int k, int lane, float dr = 0.f) {
-  if (k >= nt.n) return 0.f;
-  const T* src = static_cast<const T*>(a.src);
-  T* dst = static_cast<T*>(a.dst);
-  const LaneDir d = lane_dir(lane);
-  const uint32_t t = static_cast<uint32_t>(nt.cells[k]);
-  const uint32_t mask = nt.mask[k];
-  const uint8_t fl = a.flags[t];
-  const int sl = d.act ? nt.slot[lane * nt.n + k] : 0;
-  const float q = d.act ? nt.q[lane * nt.n + k] : 1.f, add = d.act ? nt.add[lane * nt.n + k] : 0.f;
-  pdl_wait();
-  const float val = d.act ? pull_value(a, src, lane, sl) : 0.f;
-  const float own = d.act ? LD(src, a.qs, lane, t, a.inv_scale) : 0.f;
-  const float own_opp = __shfl_sync(0xffffffffu, own, d.opp);
-  float f = val;
-  if (d.act && ((mask >> lane) & 1u)) f = (q < 1.0f ? bouzidi(own_opp, val, own, q) : own_opp) + add;
-  if ((fl & kFlagSave) && d.act) a.save_buf[static_cast<long long>(a.save_idx[t]) * kQ + lane] = f;
-  float dh = 0.f;
-  if constexpr (CM != kCollNone) {
-    if ((fl & kKindMask) == kBulk) {
-      float fa[kQ];
-      gather_lanes(f, fa);
-      if constexpr (CM == kCollConstRho) {
-        f = bgk_lane_const_rho(d, lane, fa, f, a.omega, dr, dh);
-        if (fl & kFlagProlong) dh = 0.f;
-      } else {
-        f = bgk_lane<false>(d, lane, fa, f, a.omega);
-      }
-    }
-  }
-  if (d.act) Store<T>::st(dst + lane * a.qs + t, f, a.scale);
-  return dh;
-}
-
 template <typename T, int CM = kCollBgk>
 __global__ void __launch_bounds__(kThreads) k_step_near(const StepArgs a, const NearTables nt) {
   near_cell<T, CM>(a, nt, (blockIdx.x * kThreads + threadIdx.x) >> 5, threadIdx.x & 31);
@@ -289,160 +218,6 @@ template <> struct Pair<__half> {
     *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
   }
 };
-
-// Forest-level step with a per-block slot map: one CTA per block stages the
-// block's (n+2)^3 map (padded position -> slot: own core, the neighbour core
-// the same-level exchange copies, the source cell of an outflow ghost copy,
-// the own halo page, or a bounce-back wall marker) in shared memory, so
-// every pull is one shared-memory read and one 32-bit offset, with no
-// per-direction branching at block faces.  Each thread takes cells tl and
-// tl + 256 together (n^3 a multiple of 512), all 38 pulls issued before the
-// two collisions.  Same arithmetic as k_step; kFlagNear cells are left to
-// k_step_near, solid cells of the links rule are copied.  CTAs after the
-// nblk block CTAs stream the open blocks' halo items.
-template <typename T, bool LINKS, bool FLAGS>
-__device__ __forceinline__ bool map_cell_prologue(const StepArgs& a, uint32_t t, const T* src, T* dst, uint8_t& fl) {
-  fl = FLAGS ? a.flags[t] : 0;
-  if constexpr (LINKS) {
-    if ((fl & kKindMask) == kSolid) {
-      // Solid cells are neither streamed nor collided (block_lattice.cpp:581-583).
-      copy_cell(src, dst, a.qs, t);
-      return false;
-    }
-    if (fl & kFlagNear) return false;
-  }
-  return true;
-}
-
-template <typename T, bool FLAGS, int CM = kCollBgk>
-__device__ __forceinline__ float map_cell_finish(const StepArgs& a, uint32_t t, uint8_t fl, float (&f)[kQ], T* dst,
-                                                 float dr = 0.f) {
-  float dh = 0.f;
-  bool bulk = true;
-  if constexpr (FLAGS) {
-    if (fl & kFlagSave) {
-      float* sv = a.save_buf + static_cast<long long>(a.save_idx[t]) * kQ;
-#pragma unroll
-      for (int i = 0; i < kQ; ++i) sv[i] = f[i];
-    }
-    bulk = (fl & kKindMask) == kBulk;
-  }
-  if (bulk) {
-    if constexpr (CM == kCollConstRho) {
-      dh = bgk_const_rho(f, a.omega, dr);
-      if (fl & kFlagProlong) dh = 0.f;
-    } else if constexpr (CM == kCollBgk) {
-      bgk<false>(f, a.omega);
-    }
-  }
-  const uint32_t qs = static_cast<uint32_t>(a.qs);
-#pragma unroll
-  for (int i = 0; i < kQ; ++i) Store<T>::st(dst + (static_cast<uint32_t>(i) * qs + t), f[i], a.scale);
-  return dh;
-}
-
-// With one cell per thread (CPT = 1) two CTAs share a block, each over half
-// its cells, so small levels still give every SM work.  Under the links rule
-// the first CTAs of the launch take the near-wall cells (one warp each), so
-// they run beside the bulk instead of in a launch of their own.
-//
-// CM = kCollConstRho: the ConstRhoBGK collide at average density *cr_avg,
-// and per near-cell and block CTA the sum of rho - 1 over its collided kBulk
-// cells in cr_part[blockIdx.x] (the halo-item CTAs after them write none);
-// kCollNone: no collide.
-template <typename T, bool LINKS, bool FLAGS, int CPT, bool GMAP, int CM = kCollBgk>
-__global__ void __launch_bounds__(kThreads, CPT == 2 ? 4 : 5) k_step_map(const StepArgs a, const NearTables nt) {
-  extern __shared__ int smap_s[];  // (n+2)^3 slots of this block
-  constexpr uint32_t kParts = CPT == 1 ? 2 : 1;
-  const uint32_t near_ctas = LINKS ? (static_cast<uint32_t>(nt.n) + kThreads / 32 - 1) / (kThreads / 32) : 0;
-  if (LINKS && blockIdx.x < near_ctas) {
-    if constexpr (CM == kCollConstRho) {
-      pdl_wait();
-      const float dr = static_cast<float>(1.0 - *a.cr_avg);
-      const float dh = near_cell<T, kCollConstRho>(a, nt, static_cast<int>(blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)),
-                                          threadIdx.x & 31, dr);
-      cr_store_partial(a, (threadIdx.x & 31) == 0 ? static_cast<double>(dh) : 0.0,
-                       near_ctas + static_cast<uint32_t>(a.nblk) * kParts);
-    } else {
-      near_cell<T, CM>(a, nt, static_cast<int>(blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5)), threadIdx.x & 31);
-    }
-    return;
-  }
-  const uint32_t bid = blockIdx.x - near_ctas;
-  const uint32_t b = bid / kParts, part = bid % kParts;
-  if (b >= static_cast<uint32_t>(a.nblk)) {
-    pdl_wait();
-    rotate_item<T>(a, (bid - a.nblk * kParts) * kThreads + threadIdx.x);
-    return;
-  }
-  const int np = a.np, np3 = np * np * np;
-  const int* gm = a.slot_map + static_cast<long long>(b) * np3;
-  if constexpr (!GMAP) {
-    for (int k = threadIdx.x; k < np3; k += kThreads) smap_s[k] = gm[k];
-    __syncthreads();
-  }
-  // GMAP: the map is read through the read-only L1 path instead (no staging
-  // barrier); 4 KB per block stays L1-resident for the CTA
-  const int* smap = GMAP ? gm : smap_s;
-  const bool moving = a.blk_moving[b] != 0;  // uniform over the CTA
-  pdl_wait();
-  const T* src = static_cast<const T*>(a.src);
-  T* dst = static_cast<T*>(a.dst);
-  const uint32_t n = a.n, n3 = n * n * n, qs = static_cast<uint32_t>(a.qs);
-  const uint32_t span = n3 / kParts;
-  const float dr = CM == kCollConstRho ? static_cast<float>(1.0 - *a.cr_avg) : 0.f;
-  float acc = 0.f;
-  for (uint32_t tl0 = part * span + threadIdx.x; tl0 < (part + 1) * span; tl0 += CPT * kThreads) {
-    uint32_t t[CPT];
-    int P[CPT];
-    uint8_t fl[CPT];
-    bool go[CPT];
-    float f[CPT][kQ];
-#pragma unroll
-    for (int c = 0; c < CPT; ++c) {
-      const uint32_t tl = tl0 + c * kThreads;
-      t[c] = b * n3 + tl;
-      const uint32_t x = a.div_n2.div(tl), r = tl - x * n * n, y = a.div_n.div(r);
-      P[c] = (static_cast<int>(x + 1) * np + static_cast<int>(y + 1)) * np + static_cast<int>(r - y * n + 1);
-      go[c] = map_cell_prologue<T, LINKS, FLAGS>(a, t[c], src, dst, fl[c]);
-    }
-#pragma unroll
-    for (int i = 0; i < kQ; ++i) {
-      const uint32_t row = static_cast<uint32_t>(i) * qs;
-#pragma unroll
-      for (int c = 0; c < CPT; ++c) {
-        // bounce-back wall position (marker < 0): the cell's own opposite
-        // population; branch-free so the 19 (or 38) loads stay independent
-        const int sm = GMAP ? __ldg(smap + P[c] - a.off_pad[i]) : smap[P[c] - a.off_pad[i]];
-        const uint32_t off = sm >= 0 ? row + static_cast<uint32_t>(sm) : static_cast<uint32_t>(opp(i)) * qs + t[c];
-        const float v = Store<T>::ld(src + off, a.inv_scale);
-        // two cells per thread: the moving-wall term inline (a separate pass
-        // costs these variants registers)
-        if constexpr (CPT == 2) f[c][i] = sm < -1 ? v + a.wall_add[(-sm - 2) * kQ + i] : v;
-        else f[c][i] = v;
-      }
-    }
-    if (CPT == 1 && moving) {
-      // moving-wall markers (< -1) add the wall term: only blocks flagged in
-      // blk_moving hold one, the others skip this pass
-#pragma unroll
-      for (int i = 0; i < kQ; ++i)
-#pragma unroll
-        for (int c = 0; c < CPT; ++c) {
-          const int sm = GMAP ? __ldg(smap + P[c] - a.off_pad[i]) : smap[P[c] - a.off_pad[i]];
-          if (sm < -1) f[c][i] += a.wall_add[(-sm - 2) * kQ + i];
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < CPT; ++c)
-      if (go[c]) {
-        if constexpr (CM == kCollConstRho) acc += map_cell_finish<T, FLAGS, CM>(a, t[c], fl[c], f[c], dst, dr);
-        else map_cell_finish<T, FLAGS, CM>(a, t[c], fl[c], f[c], dst);
-      }
-  }
-  if constexpr (CM == kCollConstRho)
-    cr_store_partial(a, static_cast<double>(acc), near_ctas + static_cast<uint32_t>(a.nblk) * kParts);
-}
 
 // One periodic all-kBulk block, two consecutive z cells per thread: every
 // population row is read and written with 2-element vector accesses; a z-shift
@@ -1191,61 +966,9 @@ cudaError_t launch_step(const StepArgs& a, bool periodic, bool links, bool flags
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// Slot-map step: a CTA of 256 threads per block (n^3 a multiple of 512, the
-// (n+2)^3 map within 48 KB of shared memory, 32-bit population offsets).
-bool map_step_eligible(int n, long long nslots) {
-  const long long np = n + 2;
-  return n % 8 == 0 && np * np * np * 4 <= 48 * 1024 && nslots * kQ < (1LL << 32);
-}
-template <typename T>
-cudaError_t launch_step_map(const StepArgs& a, const NearTables& nt, bool links, bool flags, int cpt, bool gmap,
-                            cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
-  if (a.nitems == 0) return cudaSuccess;
-  const uint32_t near_ctas = links ? grid_for(static_cast<uint32_t>(nt.n) * 32) : 0;
-  const dim3 g(near_ctas + static_cast<uint32_t>(a.nblk) * (cpt == 2 ? 1 : 2) + grid_for(static_cast<uint32_t>(a.n_open)));
-  const size_t smem = gmap ? 0 : static_cast<size_t>(a.np) * a.np * a.np * sizeof(int);
-#define OCTLB_MAP_LAUNCH(C, G)                                                                              \
-  if (links) e = launch_chain(k_step_map<T, true, true, C, G>, g, dim3(kThreads), smem, s, a, nt);          \
-  else if (flags) e = launch_chain(k_step_map<T, false, true, C, G>, g, dim3(kThreads), smem, s, a, nt);    \
-  else e = launch_chain(k_step_map<T, false, false, C, G>, g, dim3(kThreads), smem, s, a, nt);
-  if (cpt == 2) {
-    if (gmap) { OCTLB_MAP_LAUNCH(2, true) } else { OCTLB_MAP_LAUNCH(2, false) }
-  } else {
-    if (gmap) { OCTLB_MAP_LAUNCH(1, true) } else { OCTLB_MAP_LAUNCH(1, false) }
-  }
-#undef OCTLB_MAP_LAUNCH
-  return e != cudaSuccess ? e : cudaGetLastError();
-}
-
-// ConstRhoBGK slot-map step: the default variants only (one cell per thread
-// under the links rule, two otherwise; slot map read through L1).
-template <typename T>
-cudaError_t launch_step_map_cr(const StepArgs& a, const NearTables& nt, bool links, bool flags, cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
-  if (a.nitems == 0) return cudaSuccess;
-  const uint32_t near_ctas = links ? grid_for(static_cast<uint32_t>(nt.n) * 32) : 0;
-  const dim3 g(near_ctas + static_cast<uint32_t>(a.nblk) * (links ? 2 : 1) + grid_for(static_cast<uint32_t>(a.n_open)));
-  if (links) e = launch_chain(k_step_map<T, true, true, 1, true, kCollConstRho>, g, dim3(kThreads), 0, s, a, nt);
-  else if (flags) e = launch_chain(k_step_map<T, false, true, 2, true, kCollConstRho>, g, dim3(kThreads), 0, s, a, nt);
-  else e = launch_chain(k_step_map<T, false, false, 2, true, kCollConstRho>, g, dim3(kThreads), 0, s, a, nt);
-  return e != cudaSuccess ? e : cudaGetLastError();
-}
-
-// Stream-only steps (no collide) of the levels above the finest under
-// ConstRhoBGK on a multi-level mesh: the slot-map form in the variants of
-// launch_step_map_cr, else the core / halo-item launch and the near cells.
-template <typename T>
-cudaError_t launch_step_map_nc(const StepArgs& a, const NearTables& nt, bool links, bool flags, cudaStream_t s) {
-  cudaError_t e = cudaSuccess;
-  if (a.nitems == 0) return cudaSuccess;
-  const uint32_t near_ctas = links ? grid_for(static_cast<uint32_t>(nt.n) * 32) : 0;
-  const dim3 g(near_ctas + static_cast<uint32_t>(a.nblk) * (links ? 2 : 1) + grid_for(static_cast<uint32_t>(a.n_open)));
-  if (links) e = launch_chain(k_step_map<T, true, true, 1, true, kCollNone>, g, dim3(kThreads), 0, s, a, nt);
-  else if (flags) e = launch_chain(k_step_map<T, false, true, 2, true, kCollNone>, g, dim3(kThreads), 0, s, a, nt);
-  else e = launch_chain(k_step_map<T, false, false, 2, true, kCollNone>, g, dim3(kThreads), 0, s, a, nt);
-  return e != cudaSuccess ? e : cudaGetLastError();
-}
+// Stream-only step (no collide) of a level above the finest under ConstRhoBGK
+// on a multi-level mesh, where the slot-map step does not run: the core /
+// halo-item launch and the near cells.
 template <typename T>
 cudaError_t launch_step_nc(const StepArgs& a, const NearTables& nt, bool links, bool flags, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
@@ -1436,7 +1159,6 @@ cudaError_t launch_cr_update(double* avg, const double* part, int nparts, long l
   template cudaError_t launch_step_aa<T>(const StepArgs&, bool, cudaStream_t);                     \
   template cudaError_t launch_step_near<T>(const StepArgs&, const NearTables&, cudaStream_t);       \
   template cudaError_t launch_add_force<T>(const StepArgs&, T*, const float*, cudaStream_t);         \
-  template cudaError_t launch_step_map<T>(const StepArgs&, const NearTables&, bool, bool, int, bool, cudaStream_t); \
   template cudaError_t launch_couple<T>(const ProlongOp&, const RestrictOp&, const RestrictOp&,    \
                                         cudaStream_t);                                             \
   template cudaError_t launch_drag<T>(const StepArgs&, bool, const DragItem*, int, double*,        \
@@ -1446,8 +1168,6 @@ cudaError_t launch_cr_update(double* avg, const double* part, int nparts, long l
   template cudaError_t launch_scatter<T>(const StepArgs&, const double*, int, cudaStream_t);     \
   template cudaError_t launch_scatter_eq<T>(const StepArgs&, const double*, int, cudaStream_t);  \
   template cudaError_t launch_step_cr<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
-  template cudaError_t launch_step_map_cr<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
-  template cudaError_t launch_step_map_nc<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
   template cudaError_t launch_step_nc<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
   template cudaError_t launch_collide_cr<T>(const StepArgs&, float*, cudaStream_t);                \
   template cudaError_t launch_cr_seed<T>(const StepArgs&, int, cudaStream_t);

@@ -150,8 +150,8 @@ int launch_level_step(octlb_ctx* ctx, Level& L) {
     // collide gives (the stored state of every level is again one collide
     // ahead after advance_one)
     const bool links = ctx->stream_mode == OCTLB_STREAM_LINKS;
-    if (L.use_map && ctx->map_global && ctx->map_cells == (links ? 1 : 2)) {
-      CK(launch_step_map_nc<T>(a, L.near, links, L.has_flags, ctx->stream));
+    if (L.use_map) {
+      CK(launch_step_map<T>(a, L.near, links, L.has_flags, kCollNone, ctx->stream));
     } else {
       CK(launch_step_nc<T>(a, L.near, links, L.has_flags, ctx->stream));
       if (L.near.n > 0) ++ctx->launch_count;
@@ -165,8 +165,8 @@ int launch_level_step(octlb_ctx* ctx, Level& L) {
                         ctx->cr_count, ctx->fd_cr_part.as<double>(), ctx->fd_cr_parts, ctx->fd_vel,
                         ctx->cr_shift.as<float>() + L.lvl, ctx->stream));
     const bool links = ctx->stream_mode == OCTLB_STREAM_LINKS;
-    if (L.use_map && ctx->map_global && ctx->map_cells == (links ? 1 : 2)) {
-      CK(launch_step_map_cr<T>(a, L.near, links, L.has_flags, ctx->stream));
+    if (L.use_map) {
+      CK(launch_step_map<T>(a, L.near, links, L.has_flags, kCollConstRho, ctx->stream));
       ++ctx->launch_count;
     } else {
       CK(launch_step_cr<T>(a, L.near, links, L.has_flags, ctx->stream));
@@ -185,8 +185,7 @@ int launch_level_step(octlb_ctx* ctx, Level& L) {
   } else if (L.use_pair) {
     CK(launch_step_pair<T>(a, ctx->stream));
   } else if (L.use_map) {
-    CK(launch_step_map<T>(a, L.near, ctx->stream_mode == OCTLB_STREAM_LINKS, L.has_flags, ctx->map_cells,
-                          ctx->map_global, ctx->stream));
+    CK(launch_step_map<T>(a, L.near, ctx->stream_mode == OCTLB_STREAM_LINKS, L.has_flags, kCollBgk, ctx->stream));
   } else {
     CK(launch_step<T>(a, ctx->periodic != 0, ctx->stream_mode == OCTLB_STREAM_LINKS, L.has_flags,
                       ctx->stream));
@@ -654,6 +653,12 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
   // ---- per-level flags, links, neighbour bases, halo pages, boundary fills,
   //      drag items
   const int np = n + 2, np3 = np * np * np;
+  int sms = 0;
+  if (!g_dry_run) {
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
   // Velocity scale of the moving tree-boundary walls (the largest wall speed,
   // e.g. the inlet u_max): every wall velocity is taken proportional to it
   // for the adjoint's d/du_max.
@@ -664,16 +669,19 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
       wall_vscale = std::max(wall_vscale, std::sqrt(sp[1] * sp[1] + sp[2] * sp[2] + sp[3] * sp[3]));
   }
   ctx->wall_vscale = wall_vscale;
+  // Halo index of every padded position outside the core: first the z rows of
+  // the x and y faces and of the x-y edges (n positions each, so the rows of an
+  // even n start on even slots), then the rest.
   std::vector<int> hmap(static_cast<size_t>(np3), -1), hpos;
-  for (int X = 0; X < np; ++X)
-    for (int Y = 0; Y < np; ++Y)
-      for (int Z = 0; Z < np; ++Z) {
-        const bool core = X >= 1 && Y >= 1 && Z >= 1 && X <= n && Y <= n && Z <= n;
-        if (!core) {
+  for (int pass = 0; pass < 2; ++pass)
+    for (int X = 0; X < np; ++X)
+      for (int Y = 0; Y < np; ++Y)
+        for (int Z = 0; Z < np; ++Z) {
+          const bool core = X >= 1 && Y >= 1 && Z >= 1 && X <= n && Y <= n && Z <= n;
+          if (core || (Z >= 1 && Z <= n) != (pass == 0)) continue;
           hmap[(X * np + Y) * np + Z] = static_cast<int>(hpos.size());
           hpos.push_back((X * np + Y) * np + Z);
         }
-      }
   const int H = static_cast<int>(hpos.size());
   auto dir27 = [&](int X, int Y, int Z) {
     const int ox = X == 0 ? -1 : (X == n + 1 ? 1 : 0), oy = Y == 0 ? -1 : (Y == n + 1 ? 1 : 0),
@@ -1052,8 +1060,8 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
             nmask[k] |= 1u << i;
             if (li >= 0) {
               const float q = lrec[static_cast<size_t>(li) * 38 + i];
-              nq[i * nn + k] = q;
-              nadd[i * nn + k] = lrec[static_cast<size_t>(li) * 38 + kQ + i];
+              nq[k * kQ + i] = q;
+              nadd[k * kQ + i] = lrec[static_cast<size_t>(li) * 38 + kQ + i];
               if (q < 1.0f) {
                 // f_q: population i of x + c_i when that cell is kBulk (a halo
                 // position counts as kBulk), else the cell's own
@@ -1067,7 +1075,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
             }
           }
           if (sl >= (1LL << 31)) return fail(ctx, OCTLB_EINVAL, "level has more than 2^31 slots");
-          nslot[i * nn + k] = static_cast<int>(sl);
+          nslot[k * kQ + i] = static_cast<int>(sl);
         }
       }
     }
@@ -1206,6 +1214,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     A.n_open = L.n_open;
     A.n_halo = L.n_halo;
     A.nblk = L.nblk; A.n = n; A.np = np;
+    A.sms = sms;
     A.halo_base = core_end;
     A.ncore = static_cast<uint32_t>(ncore);
     A.nitems = A.ncore + static_cast<uint32_t>(L.n_open);
@@ -1244,12 +1253,32 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
       CK(upload(L.slot_map, slot_map));
       CK(upload(L.wall_add, wall_add));
       CK(upload(L.wall_dadd, wall_dadd));
-      std::vector<uint8_t> moving(static_cast<size_t>(L.nblk), 0);
-      for (int lb = 0; lb < L.nblk; ++lb)
-        for (int k = 0; k < np3 && !moving[lb]; ++k)
-          if (slot_map[static_cast<size_t>(lb) * np3 + k] < -1) moving[lb] = 1;
-      CK(upload(L.blk_moving, moving));
-      A.blk_moving = L.blk_moving.as<uint8_t>();
+      std::vector<uint8_t> info(static_cast<size_t>(L.nblk), kBlkRows);
+      std::vector<int> row_map(static_cast<size_t>(L.nblk) * 3 * np * np);
+      for (int lb = 0; lb < L.nblk; ++lb) {
+        const int* m = slot_map.data() + static_cast<size_t>(lb) * np3;
+        for (int r = 0; r < np * np; ++r)
+          for (int k = 0; k < 3; ++k)
+            row_map[(static_cast<size_t>(lb) * 3 + k) * np * np + r] = m[r * np + (k == 0 ? 1 : (k == 1 ? 0 : np - 1))];
+        for (int k = 0; k < np3; ++k)
+          if (m[k] < -1) info[lb] |= kBlkMoving;
+        for (int X = 0; X < np; ++X)
+          for (int Y = 0; Y < np; ++Y) {
+            const int* r = m + (X * np + Y) * np;
+            const bool edge = (X == 0 || X == np - 1) && (Y == 0 || Y == np - 1);
+            bool wall = r[1] < 0, run = (r[1] & 1) == 0, same = edge && (r[1] & 1) == 0 && r[1] >= 0;
+            for (int Z = 1; Z <= n; ++Z) {
+              wall = wall && (r[1] == -1 ? r[Z] == -1 : r[Z] == r[1] - (Z - 1));
+              run = run && r[Z] >= 0 && r[Z] == r[1] + Z - 1;
+              same = same && r[Z] == r[1];  // an edge row nothing resolves (never pulled by a streamed cell)
+            }
+            if (!wall && !run && !same) info[lb] &= static_cast<uint8_t>(~kBlkRows);
+          }
+      }
+      CK(upload(L.blk_info, info));
+      CK(upload(L.row_map, row_map));
+      A.row_map = L.row_map.as<int>();
+      A.blk_info = L.blk_info.as<uint8_t>();
       A.slot_map = L.slot_map.as<int>();
       A.wall_add = L.wall_add.as<float>();
       A.wall_dadd = L.wall_dadd.as<float>();
@@ -1259,9 +1288,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     if (L.use_pair && sizeof(T) == 2 && ctx->fp16_rows >= 0 &&
         rows_step_eligible(n, L.ncore, L.nslots, ctx->fp16_rows) && !g_dry_run) {
       const int per_sm = rows_prepare(ctx->fp16_rows, false);
-      int dev = 0, sms = 0;
-      CK(cudaGetDevice(&dev));
-      CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (per_sm > 0) {
         L.use_rows = true;
         L.rows_grid = static_cast<int>(std::min<long long>(static_cast<long long>(per_sm) * sms,
@@ -1273,9 +1299,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     if (L.aa && ctx->aa_rows >= 0 && aa_rows_eligible(n, L.ncore, L.nslots, sizeof(T), ctx->aa_rows) &&
         !g_dry_run) {
       const int per_sm = aa_rows_prepare<T>(ctx->aa_rows);
-      int dev = 0, sms = 0;
-      CK(cudaGetDevice(&dev));
-      CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (per_sm > 0) {
         L.use_aa_rows = true;
         L.aa_rows_grid = static_cast<int>(std::min<long long>(static_cast<long long>(per_sm) * sms,
@@ -1286,9 +1309,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     if (L.aa && sizeof(T) == 2 && ctx->fp16_rows >= 0 && rows_step_eligible(n, L.ncore, L.nslots, ctx->fp16_rows) &&
         !g_dry_run) {
       const int per_sm = rows_prepare(ctx->fp16_rows, true);
-      int dev = 0, sms = 0;
-      CK(cudaGetDevice(&dev));
-      CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (per_sm > 0) {
         L.use_aa_local_rows = true;
         L.aa_local_grid = static_cast<int>(std::min<long long>(static_cast<long long>(per_sm) * sms,
@@ -1297,9 +1317,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     }
     if (uniform && ctx->step_kernel == 1 && bulk_step_eligible(n, sizeof(T)) && !g_dry_run) {
       const int per_sm = bulk_prepare<T>(n);
-      int dev = 0, sms = 0;
-      CK(cudaGetDevice(&dev));
-      CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (per_sm > 0) {
         L.use_bulk = true;
         L.bulk_grid = std::min(per_sm * sms, n * n);
@@ -2153,9 +2170,6 @@ static int create_common(const octlb_tables* t, const octlb_params* p, const dou
     const std::string v(sk);
     ctx->step_kernel = v == "bulk" ? 1 : (v == "plain" ? 2 : 0);
   }
-  ctx->map_cells = p->stream_mode == OCTLB_STREAM_LINKS ? 1 : 2;
-  if (const char* mc = std::getenv("OCTLB_MAP_CELLS")) ctx->map_cells = mc[0] == '1' ? 1 : 2;
-  if (const char* ms = std::getenv("OCTLB_MAP_SMEM")) ctx->map_global = ms[0] != '1';
   if (const char* wm = std::getenv("OCTLB_WAIT_MS")) {
     const long long ms = std::atoll(wm);
     if (ms >= 1 && ms <= 60000) ctx->wait_ns = static_cast<unsigned long long>(ms) * 1000000ull;

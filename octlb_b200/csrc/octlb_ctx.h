@@ -37,10 +37,6 @@ template <typename T>
 cudaError_t launch_step_cr(const StepArgs&, const NearTables&, bool, bool, cudaStream_t);
 template <typename T> cudaError_t launch_cr_seed(const StepArgs&, int, cudaStream_t);
 template <typename T>
-cudaError_t launch_step_map_cr(const StepArgs&, const NearTables&, bool, bool, cudaStream_t);
-template <typename T>
-cudaError_t launch_step_map_nc(const StepArgs&, const NearTables&, bool, bool, cudaStream_t);
-template <typename T>
 cudaError_t launch_step_nc(const StepArgs&, const NearTables&, bool, bool, cudaStream_t);
 template <typename T> cudaError_t launch_collide_cr(const StepArgs&, float*, cudaStream_t);
 template <typename T> cudaError_t launch_step_aa(const StepArgs&, bool, cudaStream_t);
@@ -62,7 +58,7 @@ template <typename T> cudaError_t launch_step_aa_rows(const StepArgs&, int varia
 template <typename T> cudaError_t launch_step_pair(const StepArgs&, cudaStream_t);
 template <typename T> cudaError_t launch_step_near(const StepArgs&, const NearTables&, cudaStream_t);
 template <typename T> cudaError_t launch_add_force(const StepArgs&, T*, const float*, cudaStream_t);
-template <typename T> cudaError_t launch_step_map(const StepArgs&, const NearTables&, bool, bool, int, bool, cudaStream_t);
+template <typename T> cudaError_t launch_step_map(const StepArgs&, const NearTables&, bool, bool, int, cudaStream_t);
 bool pair_step_eligible(int n);
 bool map_step_eligible(int n, long long nslots);
 void set_programmatic_launch(bool on);
@@ -152,7 +148,7 @@ struct Level {
   DevBuf buf[2];
   int cur = 0;
   DevBuf flags, link_idx, link_rec, save_idx, save_buf;
-  DevBuf nbase, page_of, hmap, hpos, open_pages, near_cells, slot_map;
+  DevBuf nbase, page_of, hmap, hpos, open_pages, near_cells, slot_map, row_map;
   DevBuf near_mask, near_slot, near_q, near_add;
   NearTables near{};
   int n_near = 0;
@@ -162,7 +158,7 @@ struct Level {
   // tree-boundary halo fills
   DevBuf bb_ops, fill_of;           // fills, and per (page slot, population) the fill index or -1
   DevBuf wall_add, wall_dadd;       // slot-map wall markers' terms
-  DevBuf blk_moving;                // per block: its map holds a moving-wall marker
+  DevBuf blk_info;                  // per block: what its map holds (kBlkMoving, kBlkRows)
   uint32_t n_bb = 0;
   // coupler: this level as coarse (prolong) and as fine (restrict)
   DevBuf prolong_items, prev, restrict_items;
@@ -330,7 +326,6 @@ struct octlb_ctx {
   int step_kernel = 0;              // OCTLB_STEP_KERNEL: 0 pair (default), 1 bulk, 2 plain
   int fp16_rows = 0;                // OCTLB_FP16_ROWS: the staged FP16 step's launch shape (off: -1)
   int aa_rows = 0;                  // OCTLB_AA_ROWS: the staged AA pull step's launch shape (off: -1)
-  bool map_global = true;           // slot map read through L1 (OCTLB_MAP_SMEM=1: staged in shared memory)
   // Bounded device waits: their limit (OCTLB_WAIT_MS, default 1 s) and the
   // test of the give-up path (OCTLB_TEST_BULK_STALL=1: one CTA of the bulk
   // step waits for a row it never requested).  After a give-up whose own
@@ -338,8 +333,6 @@ struct octlb_ctx {
   unsigned long long wait_ns = 1000000000ull;
   int stall_first_row = 0;
   bool unusable = false;
-  int map_cells = 0;                // cells per thread of the slot-map step (OCTLB_MAP_CELLS 1 or 2;
-                                    // default 2, 1 under the links rule whose variant spills at 2)
   // advance_one captured as CUDA graphs, keyed by the A/B parity of every
   // level's buffers (the launch arguments depend on it)
   struct GraphEntry {

@@ -35,13 +35,15 @@ struct StepArgs {
   const int* hpos;          // [n_halo] halo index -> padded linear position
   const int* open_pages;    // [n_open][4] torus-streamed halo items: page, block, halo index, population
   const int* slot_map;      // [nblk][(n+2)^3] slot of every padded position (k_step_map levels)
+  const int* row_map;       // [nblk][3][(n+2)^2] slot map at Z = 1, 0 and n + 1 (kBlkRows blocks)
   const int* fill_of;       // [n_pages * n_halo][19] boundary fill writing (page slot, population), or -1
   const struct BBOp* fills; // the fills (never materialised: readers take the source, pull_value)
   const float* wall_add;    // [k][19] wall terms of slot-map marker -(2 + k) (moving bounce-back wall)
   const float* wall_dadd;   // [k][19] their derivative by the wall-velocity scale
-  const uint8_t* blk_moving; // [nblk] 1 where the block's slot map holds a moving-wall marker
+  const uint8_t* blk_info;  // [nblk] kBlkMoving, kBlkRows
   int n_open, n_halo;       // items, halo slots per page
   int nblk, n, np;          // np = n + 2
+  int sms;                  // SMs of the device
   long long halo_base;      // first halo-page slot (= nblk * n^3)
   uint32_t ncore;           // nblk * n^3 core work items
   uint32_t nitems;          // ncore + n_open
@@ -80,7 +82,8 @@ __device__ __forceinline__ long long aa_rev_slot(const StepArgs& a, int i, uint3
 }
 
 // Cells flagged kFlagNear with the link rule resolved on the host: for near
-// cell k and direction i (arrays [kQ][n]), the slot whose population i the
+// cell k and direction i (arrays [n][kQ]: a warp reads its cell's 19 entries
+// side by side), the slot whose population i the
 // rule reads (the pull source, the Bouzidi neighbour x + c_i, or the cell
 // itself), and for directions set in mask[k] the link coefficients q (1 =
 // half-way bounce-back) and the added moving-wall term (-0 when the cell has
@@ -88,11 +91,17 @@ __device__ __forceinline__ long long aa_rev_slot(const StepArgs& a, int i, uint3
 struct NearTables {
   const int* cells;         // [n] core slot
   const uint32_t* mask;     // [n] bit i: direction i takes the link rule
-  const int* slot;          // [kQ][n]
-  const float* q;           // [kQ][n]
-  const float* add;         // [kQ][n]
+  const int* slot;          // [n][kQ]
+  const float* q;           // [n][kQ]
+  const float* add;         // [n][kQ]
   int n;
 };
+
+// What a block's slot map holds: kBlkMoving a moving-wall marker; kBlkRows
+// only uniform z rows: the positions Z = 1..n of every (X, Y) are n adjacent
+// slots from an even one, or all wall markers (all -1, or n consecutive moving
+// ones, descending).
+enum : uint8_t { kBlkMoving = 1, kBlkRows = 2 };
 
 constexpr long long kOwnPage = -(1LL << 62);
 
