@@ -742,17 +742,29 @@ k_audit(const StepArgs a, double* partial) {
     for (int k = 0; k < 5; ++k) partial[blockIdx.x * 5 + k] = acc[k];
 }
 
+// Cell t of the level in the host arrays: block-local order kept, its block at
+// gid[block] (null: the level's blocks are the arrays' blocks in order).  With
+// gid a forest's levels go to and come from one array in the caller's block
+// order, and one copy moves it: reordering on the host cost 40 ms of a 512x128x
+// 128 cylinder's get_fields (94 MB, pageable buffers), the one copy takes 2.
+__device__ __forceinline__ long long host_cell(const StepArgs& a, const int* gid, uint32_t t) {
+  if (!gid) return t;
+  const uint32_t b = a.div_n3.div(t);
+  return static_cast<long long>(gid[b]) * (a.n * a.n * a.n) + (t - b * a.n * a.n * a.n);
+}
+
 // Core cells <-> dense FP64 host order [block][ix][iy][iz][19].
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_gather(const StepArgs a, double* out, double* out_u, int mode /*0 pops, 1 fields*/) {
+k_gather(const StepArgs a, double* out, double* out_u, const int* gid, int mode /*0 pops, 1 fields*/) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= a.ncore) return;
   const long long slot = t;  // compact core slot
+  const long long hc = host_cell(a, gid, t);
   const T* src = static_cast<const T*>(a.src);
   if (mode == 0) {
 #pragma unroll
-    for (int i = 0; i < kQ; ++i) out[static_cast<long long>(t) * kQ + i] = LDR(a, src, i, t);
+    for (int i = 0; i < kQ; ++i) out[hc * kQ + i] = LDR(a, src, i, t);
   } else {
     double drho = 0, jx = 0, jy = 0, jz = 0;
 #pragma unroll
@@ -764,10 +776,10 @@ k_gather(const StepArgs a, double* out, double* out_u, int mode /*0 pops, 1 fiel
     // ConstRhoBGK: the stored state is one collide ahead, which added
     // 1 - average_rho to the density of a kBulk cell and left u unchanged
     const bool cr = a.cr_avg && (a.flags ? (a.flags[slot] & kKindMask) : kBulk) == kBulk;
-    out[t] = cr ? rho - (1.0 - *a.cr_avg) : rho;
-    out_u[static_cast<long long>(t) * 3 + 0] = jx / rho;
-    out_u[static_cast<long long>(t) * 3 + 1] = jy / rho;
-    out_u[static_cast<long long>(t) * 3 + 2] = jz / rho;
+    out[hc] = cr ? rho - (1.0 - *a.cr_avg) : rho;
+    out_u[hc * 3 + 0] = jx / rho;
+    out_u[hc * 3 + 1] = jy / rho;
+    out_u[hc * 3 + 2] = jz / rho;
   }
 }
 
@@ -777,14 +789,15 @@ k_gather(const StepArgs a, double* out, double* out_u, int mode /*0 pops, 1 fiel
 // that collide; the near-wall partials after them, near_parts, are zeroed).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_scatter(const StepArgs a, const double* in, int near_parts) {
+k_scatter(const StepArgs a, const double* in, const int* gid, int near_parts) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   double v[1] = {0.0};
   if (t < a.ncore) {
     const long long slot = t;  // compact core slot
+    const double* hp = in + host_cell(a, gid, t) * kQ;
     float f[kQ];
 #pragma unroll
-    for (int i = 0; i < kQ; ++i) f[i] = static_cast<float>(in[static_cast<long long>(t) * kQ + i]);
+    for (int i = 0; i < kQ; ++i) f[i] = static_cast<float>(hp[i]);
     const uint8_t fl = a.flags ? a.flags[slot] : static_cast<uint8_t>(kBulk);
     if ((fl & kKindMask) == kBulk) {
       if (a.cr_avg) v[0] = (fl & kFlagProlong) ? 0.0 : bgk_const_rho(f, a.omega, static_cast<float>(1.0 - *a.cr_avg));
@@ -805,20 +818,20 @@ k_scatter(const StepArgs a, const double* in, int near_parts) {
 // Equilibrium state from macroscopic fields (BlockLattice::initialize and
 // initialize_from_material with a per-cell rho, u: block_lattice.cpp:273-285,
 // lattice_material_init.cpp:11-33): f_i = feq_i(rho, u) - w_i in FP64, then
-// the same conversion and collide as k_scatter.  in = [rho | u] (ncore, then
-// ncore x 3).  The FP64 operations are rounded one by one in the order
+// the same conversion and collide as k_scatter.  The FP64 operations are rounded one by one in the order
 // rho w_i (1 + 3 cu + 4.5 cu cu - 1.5 u.u) - w_i is written (no contraction
 // into fused multiply-adds), so the state equals k_scatter's of the same
 // equilibrium formed on the host in that order.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_scatter_eq(const StepArgs a, const double* in, int near_parts) {
+k_scatter_eq(const StepArgs a, const double* in_rho, const double* in_u, const int* gid, int near_parts) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   double v[1] = {0.0};
   if (t < a.ncore) {
     const long long slot = t;
-    const double rho = in[t];
-    const double* up = in + a.ncore + 3ll * t;
+    const long long hc = host_cell(a, gid, t);
+    const double rho = in_rho[hc];
+    const double* up = in_u + 3 * hc;
     const double ux = up[0], uy = up[1], uz = up[2];
     const double usq = __dadd_rn(__dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz));
     const double t6 = __dmul_rn(1.5, usq);
@@ -1087,18 +1100,19 @@ cudaError_t launch_audit(const StepArgs& a, double* partial, double* out, cudaSt
 uint32_t audit_partials(const StepArgs& a) { return grid_for(a.ncore); }
 
 template <typename T>
-cudaError_t launch_gather(const StepArgs& a, double* out, double* out_u, int mode, cudaStream_t s) {
-  k_gather<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, out, out_u, mode);
+cudaError_t launch_gather(const StepArgs& a, double* out, double* out_u, const int* gid, int mode, cudaStream_t s) {
+  k_gather<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, out, out_u, gid, mode);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_scatter(const StepArgs& a, const double* in, int near_parts, cudaStream_t s) {
-  k_scatter<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, in, near_parts);
+cudaError_t launch_scatter(const StepArgs& a, const double* in, const int* gid, int near_parts, cudaStream_t s) {
+  k_scatter<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, in, gid, near_parts);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_scatter_eq(const StepArgs& a, const double* in, int near_parts, cudaStream_t s) {
-  k_scatter_eq<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, in, near_parts);
+cudaError_t launch_scatter_eq(const StepArgs& a, const double* rho, const double* u, const int* gid, int near_parts,
+                              cudaStream_t s) {
+  k_scatter_eq<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, rho, u, gid, near_parts);
   return cudaGetLastError();
 }
 
@@ -1164,9 +1178,9 @@ cudaError_t launch_cr_update(double* avg, const double* part, int nparts, long l
   template cudaError_t launch_drag<T>(const StepArgs&, bool, const DragItem*, int, double*,        \
                                       cudaStream_t);                                               \
   template cudaError_t launch_audit<T>(const StepArgs&, double*, double*, cudaStream_t);           \
-  template cudaError_t launch_gather<T>(const StepArgs&, double*, double*, int, cudaStream_t);              \
-  template cudaError_t launch_scatter<T>(const StepArgs&, const double*, int, cudaStream_t);     \
-  template cudaError_t launch_scatter_eq<T>(const StepArgs&, const double*, int, cudaStream_t);  \
+  template cudaError_t launch_gather<T>(const StepArgs&, double*, double*, const int*, int, cudaStream_t);  \
+  template cudaError_t launch_scatter<T>(const StepArgs&, const double*, const int*, int, cudaStream_t); \
+  template cudaError_t launch_scatter_eq<T>(const StepArgs&, const double*, const double*, const int*, int, cudaStream_t); \
   template cudaError_t launch_step_cr<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
   template cudaError_t launch_step_nc<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
   template cudaError_t launch_collide_cr<T>(const StepArgs&, float*, cudaStream_t);                \

@@ -1170,6 +1170,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     CK(upload(L.nbase, nbase));
     CK(upload(L.page_of, page_of));
     CK(upload(L.hmap, hmap));
+    CK(upload(L.blk_gid, std::vector<int>(L.blocks.begin(), L.blocks.begin() + L.nblk)));
     CK(upload(L.hpos, hpos));
     CK(upload(L.open_pages, open_pages));
     CK(upload(L.near_cells, near_cells));
@@ -1448,7 +1449,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     CK(upload(d, dense));
     StepArgs a = L.args;
     a.dst = L.buf[L.cur].p;
-    CK(launch_scatter<T>(a, d.as<double>(), 0, ctx->stream));
+    CK(launch_scatter<T>(a, d.as<double>(), nullptr, 0, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
   }
   long long lups = 0;
@@ -1987,9 +1988,46 @@ bool contiguous(const Level& L) {
   return true;
 }
 
+// Whether set / get_populations and get_fields move all levels as one array in
+// the caller's block order, the kernels placing each level's blocks: one
+// context that owns every block, levels that are not runs of it, and staging
+// for all of it (a single level, or levels in block order, needs no reordering
+// and stages level by level; so does a forest whose whole staging does not fit).
+bool whole_array(octlb_ctx* ctx, size_t doubles_a, size_t doubles_b) {
+  if (!ctx->owner.empty()) return false;
+  bool runs = true;
+  for (const auto& L : ctx->levels) runs = runs && (L.nblk == 0 || contiguous(L));
+  if (runs) return false;
+  if (ctx->stage_a.reserve(doubles_a * sizeof(double)) == cudaSuccess &&
+      ctx->stage_b.reserve(doubles_b * sizeof(double)) == cudaSuccess)
+    return true;
+  cudaGetLastError();  // out of memory: level by level
+  ctx->stage_a.alloc(0);
+  ctx->stage_b.alloc(0);
+  return false;
+}
+
 template <typename T>
 int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
   const long long n3 = static_cast<long long>(ctx->n) * ctx->n * ctx->n;
+  const size_t all = static_cast<size_t>(ctx->n_blocks * n3);
+  if (whole_array(ctx, pops ? all * kQ : all, pops ? 0 : all * 3)) {
+    double* da = ctx->stage_a.as<double>();
+    double* db = ctx->stage_b.as<double>();
+    for (auto& L : ctx->levels) {
+      if (L.nblk == 0) continue;
+      StepArgs a = L.args;
+      a.src = L.buf[L.cur].p;
+      CK(launch_gather<T>(a, da, db, L.blk_gid.as<int>(), pops ? 0 : 1, ctx->stream));
+      if (!pops)
+        if (int rc = fd_fix_fields(ctx, L, L.blk_gid.as<int>(), da, db)) return rc;
+    }
+    CK(cudaMemcpyAsync(pops ? pops : rho, da, sizeof(double) * (pops ? all * kQ : all), cudaMemcpyDeviceToHost,
+                       ctx->stream));
+    if (!pops) CK(cudaMemcpyAsync(u, db, sizeof(double) * all * 3, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return OCTLB_OK;
+  }
   for (auto& L : ctx->levels) {
     if (L.nblk == 0) continue;
     const long long cells = L.nblk * n3;
@@ -2003,9 +2041,9 @@ int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
     StepArgs a = L.args;
     a.src = L.buf[L.cur].p;
     a.aa_rev = L.aa && L.cur;
-    CK(launch_gather<T>(a, d.as<double>(), du.as<double>(), mode, ctx->stream));
+    CK(launch_gather<T>(a, d.as<double>(), du.as<double>(), nullptr, mode, ctx->stream));
     if (mode == 1)  // the FD pass's Dirichlet cells: the fields of their rewritten rows
-      if (int rc = fd_fix_fields(ctx, L, d.as<double>(), du.as<double>())) return rc;
+      if (int rc = fd_fix_fields(ctx, L, nullptr, d.as<double>(), du.as<double>())) return rc;
     const bool direct = contiguous(L);
     const long long off = static_cast<long long>(L.blocks[0]) * n3;
     std::vector<double> h0, h1;
@@ -2037,6 +2075,19 @@ int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
 template <typename T>
 int scatter_impl(octlb_ctx* ctx, const double* in) {
   const long long n3 = static_cast<long long>(ctx->n) * ctx->n * ctx->n;
+  const size_t all = static_cast<size_t>(ctx->n_blocks * n3) * kQ;
+  if (whole_array(ctx, all, 0)) {
+    double* d = ctx->stage_a.as<double>();
+    CK(cudaMemcpyAsync(d, in, sizeof(double) * all, cudaMemcpyHostToDevice, ctx->stream));
+    for (auto& L : ctx->levels) {
+      if (L.nblk == 0) continue;
+      StepArgs a = L.args;
+      a.dst = L.buf[L.cur].p;
+      CK(launch_scatter<T>(a, d, L.blk_gid.as<int>(), a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
+    return OCTLB_OK;
+  }
   for (auto& L : ctx->levels) {
     if (L.nblk == 0) continue;
     const long long cells = L.nblk * n3;
@@ -2053,7 +2104,7 @@ int scatter_impl(octlb_ctx* ctx, const double* in) {
     }
     StepArgs a = L.args;
     a.dst = L.buf[L.cur].p;
-    CK(launch_scatter<T>(a, d.as<double>(), a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    CK(launch_scatter<T>(a, d.as<double>(), nullptr, a.cr_part ? ctx->cr_near : 0, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (L.aa) L.cur = 0;  // the natural layout again
   }
@@ -2068,6 +2119,21 @@ int scatter_impl(octlb_ctx* ctx, const double* in) {
 template <typename T>
 int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
   const long long n3 = static_cast<long long>(ctx->n) * ctx->n * ctx->n;
+  const size_t all = static_cast<size_t>(ctx->n_blocks * n3);
+  if (whole_array(ctx, all, all * 3)) {
+    double* dr = ctx->stage_a.as<double>();
+    double* du = ctx->stage_b.as<double>();
+    CK(cudaMemcpyAsync(dr, rho, sizeof(double) * all, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(du, u, sizeof(double) * 3 * all, cudaMemcpyHostToDevice, ctx->stream));
+    for (auto& L : ctx->levels) {
+      if (L.nblk == 0) continue;
+      StepArgs a = L.args;
+      a.dst = L.buf[L.cur].p;
+      CK(launch_scatter_eq<T>(a, dr, du, L.blk_gid.as<int>(), a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    }
+    CK(cudaStreamSynchronize(ctx->stream));
+    return OCTLB_OK;
+  }
   for (auto& L : ctx->levels) {
     if (L.nblk == 0) continue;
     const long long cells = L.nblk * n3;
@@ -2089,7 +2155,7 @@ int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
     }
     StepArgs a = L.args;
     a.dst = L.buf[L.cur].p;
-    CK(launch_scatter_eq<T>(a, dr, a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    CK(launch_scatter_eq<T>(a, dr, du, nullptr, a.cr_part ? ctx->cr_near : 0, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (L.aa) L.cur = 0;  // the natural layout again
   }

@@ -30,9 +30,10 @@ template <typename T>
 cudaError_t launch_drag(const StepArgs&, bool, const DragItem*, int, double*, cudaStream_t);
 cudaError_t launch_drag_total(const double*, int, double*, double*, cudaStream_t);
 template <typename T> cudaError_t launch_audit(const StepArgs&, double*, double*, cudaStream_t);
-template <typename T> cudaError_t launch_gather(const StepArgs&, double*, double*, int, cudaStream_t);
-template <typename T> cudaError_t launch_scatter(const StepArgs&, const double*, int, cudaStream_t);
-template <typename T> cudaError_t launch_scatter_eq(const StepArgs&, const double*, int, cudaStream_t);
+template <typename T> cudaError_t launch_gather(const StepArgs&, double*, double*, const int*, int, cudaStream_t);
+template <typename T> cudaError_t launch_scatter(const StepArgs&, const double*, const int*, int, cudaStream_t);
+template <typename T>
+cudaError_t launch_scatter_eq(const StepArgs&, const double*, const double*, const int*, int, cudaStream_t);
 template <typename T>
 cudaError_t launch_step_cr(const StepArgs&, const NearTables&, bool, bool, cudaStream_t);
 template <typename T> cudaError_t launch_cr_seed(const StepArgs&, int, cudaStream_t);
@@ -147,6 +148,7 @@ struct Level {
   long long ncore = 0, nslots = 0;  // core slots, core + halo-page slots
   DevBuf buf[2];
   int cur = 0;
+  DevBuf blk_gid;                   // [nblk] global block id
   DevBuf flags, link_idx, link_rec, save_idx, save_buf;
   DevBuf nbase, page_of, hmap, hpos, open_pages, near_cells, slot_map, row_map;
   DevBuf near_mask, near_slot, near_q, near_add;
@@ -422,7 +424,7 @@ int comm_nranks(const octlb_comm* comm);
 template <typename T> int fd_after_step(octlb_ctx* ctx, Level& L);
 template <typename T> int fd_before_step(octlb_ctx* ctx, Level& L);
 int fd_end_of_step(octlb_ctx* ctx);
-int fd_fix_fields(octlb_ctx* ctx, Level& L, double* rho, double* u);
+int fd_fix_fields(octlb_ctx* ctx, Level& L, const int* gid, double* rho, double* u);
 void clear_graphs(octlb_ctx* ctx);
 void comm_detach(octlb_ctx* ctx);
 
