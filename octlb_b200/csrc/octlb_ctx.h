@@ -29,7 +29,7 @@ cudaError_t launch_couple(const ProlongOp&, const RestrictOp&, const RestrictOp&
 template <typename T>
 cudaError_t launch_drag(const StepArgs&, bool, const DragItem*, int, double*, cudaStream_t);
 cudaError_t launch_drag_total(const double*, int, double*, double*, cudaStream_t);
-template <typename T> cudaError_t launch_audit(const StepArgs&, double*, double*, cudaStream_t);
+template <typename T> cudaError_t launch_audit(const StepArgs&, double*, unsigned int*, double*, cudaStream_t);
 template <typename T> cudaError_t launch_gather(const StepArgs&, double*, double*, const int*, int, cudaStream_t);
 template <typename T> cudaError_t launch_scatter(const StepArgs&, const double*, const int*, int, cudaStream_t);
 template <typename T>
@@ -316,7 +316,7 @@ struct octlb_ctx {
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   bool side_busy = false;
-  DevBuf drag_partial, force, force_sum, audit_out, audit_partial, host_tmp, dev_err;
+  DevBuf drag_partial, force, force_sum, audit_out, audit_partial, audit_done, host_tmp, dev_err;
   // FP64 host-layout staging of set/get_populations and get_fields (grown on
   // demand, kept until destroy: no allocation per call)
   DevBuf stage_a, stage_b;
