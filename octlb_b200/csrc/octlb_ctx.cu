@@ -1515,45 +1515,66 @@ struct ProgrammaticScope {
   ~ProgrammaticScope() { set_programmatic_launch(false); }
 };
 
+// `count` advance_one calls as one CUDA graph, kept by (buffer parity, count):
+// captured on first use (the host bookkeeping runs once during capture), then
+// launched.
+template <typename T>
+int advance_graph(octlb_ctx* ctx, int count) {
+  const std::pair<uint64_t, int> key{parity_mask(ctx), count};
+  auto it = ctx->graphs.find(key);
+  if (it == ctx->graphs.end()) {
+    const std::vector<int> c0 = ctx->counters_collide;
+    CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = OCTLB_OK;
+    for (int k = 0; k < count && rc == OCTLB_OK; ++k) rc = advance_one_launches<T>(ctx);
+    cudaGraph_t g = nullptr;
+    const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &g);
+    if (rc) { if (g) cudaGraphDestroy(g); return rc; }
+    if (ee != cudaSuccess) return cuda_fail(ctx, ee, "cudaStreamEndCapture");
+    octlb_ctx::GraphEntry e;
+    const cudaError_t ei = cudaGraphInstantiate(&e.exec, g, 0);
+    cudaGraphDestroy(g);
+    if (ei != cudaSuccess) return cuda_fail(ctx, ei, "cudaGraphInstantiate");
+    e.out_mask = parity_mask(ctx);
+    e.dcollide.resize(ctx->counters_collide.size());
+    for (size_t l = 0; l < e.dcollide.size(); ++l) e.dcollide[l] = ctx->counters_collide[l] - c0[l];
+    it = ctx->graphs.emplace(key, e).first;
+    CK(cudaGraphLaunch(it->second.exec, ctx->stream));
+  } else {
+    CK(cudaGraphLaunch(it->second.exec, ctx->stream));
+    for (size_t l = 0; l < ctx->levels.size(); ++l) ctx->levels[l].cur = (it->second.out_mask >> l) & 1;
+    for (size_t l = 0; l < it->second.dcollide.size(); ++l) {
+      ctx->counters_collide[l] += it->second.dcollide[l];
+      ctx->counters_stream[l] += it->second.dcollide[l];
+    }
+  }
+  if (ctx->drag) ctx->force_steps += count;
+  return OCTLB_OK;
+}
+
+// Advance_one calls per graph of a long advance: a graph launch costs the
+// stream 4 - 5 us between dependent steps, a node inside a graph under 1, so
+// short steps of few launches go sixteen to a graph (64^3 box: 9.2 us per step
+// one by one).  Steps of many launches, or long ones, gain nothing that their
+// larger capture would not cost a first pass.
+constexpr int kGraphBatch = 16;
+constexpr long long kBatchLaunches = 8, kBatchUpdates = 1LL << 22;
+
 template <typename T>
 int advance_impl(octlb_ctx* ctx, int steps) {
   const ProgrammaticScope pdl(ctx->use_pdl);
-  for (int s = 0; s < steps; ++s) {
-    if (!ctx->use_graphs) {
-      int rc = advance_one_launches<T>(ctx);
-      if (rc) return rc;
+  long long launches = 0;
+  octlb_gpu_step_stats(ctx, &launches, nullptr);
+  const bool batched = ctx->use_graphs && ctx->lups_per_step <= kBatchUpdates && launches <= kBatchLaunches;
+  for (int s = 0; s < steps;) {
+    const int count = batched && steps - s >= 2 * kGraphBatch ? kGraphBatch : 1;
+    if (ctx->use_graphs) {
+      if (int rc = advance_graph<T>(ctx, count)) return rc;
     } else {
-      const uint64_t mask = parity_mask(ctx);
-      auto it = ctx->graphs.find(mask);
-      if (it == ctx->graphs.end()) {
-        // Capture this parity's advance_one (the host bookkeeping runs once
-        // during capture), then launch it.
-        const std::vector<int> c0 = ctx->counters_collide;
-        CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = advance_one_launches<T>(ctx);
-        cudaGraph_t g = nullptr;
-        const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &g);
-        if (rc) { if (g) cudaGraphDestroy(g); return rc; }
-        if (ee != cudaSuccess) return cuda_fail(ctx, ee, "cudaStreamEndCapture");
-        octlb_ctx::GraphEntry e;
-        const cudaError_t ei = cudaGraphInstantiate(&e.exec, g, 0);
-        cudaGraphDestroy(g);
-        if (ei != cudaSuccess) return cuda_fail(ctx, ei, "cudaGraphInstantiate");
-        e.out_mask = parity_mask(ctx);
-        e.dcollide.resize(ctx->counters_collide.size());
-        for (size_t l = 0; l < e.dcollide.size(); ++l) e.dcollide[l] = ctx->counters_collide[l] - c0[l];
-        it = ctx->graphs.emplace(mask, e).first;
-        CK(cudaGraphLaunch(it->second.exec, ctx->stream));
-      } else {
-        CK(cudaGraphLaunch(it->second.exec, ctx->stream));
-        for (size_t l = 0; l < ctx->levels.size(); ++l) ctx->levels[l].cur = (it->second.out_mask >> l) & 1;
-        for (size_t l = 0; l < it->second.dcollide.size(); ++l) {
-          ctx->counters_collide[l] += it->second.dcollide[l];
-          ctx->counters_stream[l] += it->second.dcollide[l];
-        }
-      }
+      if (int rc = advance_one_launches<T>(ctx)) return rc;
+      if (ctx->drag) ++ctx->force_steps;
     }
-    if (ctx->drag) ++ctx->force_steps;
+    s += count;
   }
   return OCTLB_OK;
 }

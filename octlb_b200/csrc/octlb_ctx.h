@@ -336,13 +336,14 @@ struct octlb_ctx {
   int stall_first_row = 0;
   bool unusable = false;
   // advance_one captured as CUDA graphs, keyed by the A/B parity of every
-  // level's buffers (the launch arguments depend on it)
+  // level's buffers (the launch arguments depend on it) and the number of calls
+  // a graph holds
   struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
     uint64_t out_mask = 0;
     std::vector<int> dcollide;
   };
-  std::map<uint64_t, GraphEntry> graphs;
+  std::map<std::pair<uint64_t, int>, GraphEntry> graphs;
   bool use_graphs = true;           // OCTLB_NO_GRAPH=1 launches kernel by kernel
   bool use_pdl = true;              // OCTLB_NO_PDL=1: plain stream order between the step's kernels
   float prolong_scale = 0.f, restrict_scale = 0.f;
