@@ -258,6 +258,15 @@ __device__ inline void block_reduce(double (&v)[N]) {
   __syncthreads();  // sm is reused by the next reduction of the same width
 }
 
+// average_rho after a collide (see k_cr_update): sum = sum(rho - 1) over count
+// kBulk cells, bsum the sum of bcount boundary cells' densities.
+__device__ __forceinline__ void cr_average(double* avg, double sum, long long count, double bsum, long long bcount) {
+  if (bcount == 0)
+    *avg = count > 0 ? (2.0 - *avg) + sum / static_cast<double>(count) : 1.0;
+  else
+    *avg = (sum + static_cast<double>(count) * (2.0 - *avg) + bsum) / static_cast<double>(count + bcount);
+}
+
 // Four consecutive halves (8-byte aligned) to floats, and back with
 // round-to-nearest.
 __device__ __forceinline__ void ld4h(const __half* p, float& a, float& b, float& c, float& d) {

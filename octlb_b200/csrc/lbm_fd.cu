@@ -24,13 +24,24 @@
 // prescribed velocity of a boundary cell, the overlap padding at rest, or a
 // mirror image with flipped normal components), the density source.
 // Arithmetic FP32; storage FP32 or FP16-shifted.
-#include "octlb_internal.h"
+//
+// The launches are small and each waits for the one before, so they are
+// programmatic: every kernel lets its dependents start at once, and reads its
+// records (constant tables, two dependent reads) before it waits for its
+// predecessor, so what remains of a launch on the critical path is one read of
+// the state, the arithmetic and one write.  cavity3d's 31^3 step: 43.8 us in
+// plain stream order with a launch for the average and a store per step, 31.9 us now.
+#include "lbm_device.cuh"
 
 namespace octlb_gpu {
 
 namespace {
 
 constexpr int kFdThreads = 128;
+
+// The dependents may be launched (they wait for this grid's end before they
+// read what it writes).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // PolynomialStartScale: 10 x^3 - 15 x^4 + 6 x^5, x = t / t_end clamped to [0, 1].
 __device__ __forceinline__ float ramp(float t, float t_end) {
@@ -39,12 +50,12 @@ __device__ __forceinline__ float ramp(float t, float t_end) {
   return x * x * x * (10.f + x * (-15.f + 6.f * x));
 }
 
-__device__ __forceinline__ void prescribed(const FdCell* cells, int row, float t, float u[3]) {
-  const FdCell& b = cells[row];
-  const float r = ramp(t, b.ramp_end);
-  u[0] = r * b.u_base[0];
-  u[1] = r * b.u_base[1];
-  u[2] = r * b.u_base[2];
+// The prescribed velocity b.xyz ramped over b.w steps.
+__device__ __forceinline__ void prescribed(const float4& b, float t, float u[3]) {
+  const float r = ramp(t, b.w);
+  u[0] = r * b.x;
+  u[1] = r * b.y;
+  u[2] = r * b.z;
 }
 
 template <typename T>
@@ -105,78 +116,122 @@ __device__ __forceinline__ float w_rt(const int c[3]) {
   const int m = (c[0] != 0) + (c[1] != 0) + (c[2] != 0);
   return m == 0 ? 1.0f / 3.0f : (m == 1 ? 1.0f / 18.0f : 1.0f / 36.0f);
 }
-// Sum over the warp, every lane receiving it.
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// One boundary cell of role `role` (1 plane, 2 edge, 3 corner) per warp,
+// One boundary cell of role ROLE (1 plane, 2 edge, 3 corner) per warp,
 // lane i holding population i of every cell the stencil reads: all of them
 // are loaded up front (independent loads, one memory latency), the moments
 // and densities summed over the warp.  Rewritten populations feq(rho, u) +
 // f_neq(Pi), Pi = -rho / (3 omega) (du + du^T), into the cell's row of fnew.
-template <typename T>
+// (The corners in the last CTA of the edges' launch, in place of their own, cost
+// 8 us per step more: its rounds read their records with nothing to hide them.)
+template <typename T, int ROLE>
 __global__ void __launch_bounds__(kFdThreads)
 k_fd_reconstruct(const T* state, long long qs, float inv_s, const FdCell* cells, const int* list, int n,
-                 float* fnew, const double* time, float omega, const float* cr_shift) {
+                 float* fnew, const double* time, double time_shift, float omega, const float* cr_shift) {
+  pdl_trigger();
   const int w = static_cast<int>((blockIdx.x * kFdThreads + threadIdx.x) >> 5);
   if (w >= n) return;  // whole warps
   const int lane = threadIdx.x & 31;
   const bool act = lane < kQ;
   const int i = act ? lane : 0;
   const int ci[3] = {c_rt(0, i), c_rt(1, i), c_rt(2, i)};
+  // the cell's record, staged in shared memory before the predecessor's end
+  __shared__ __align__(16) unsigned char rec[kFdThreads / 32][(sizeof(FdCell) + 15) / 16 * 16];
   const int row = list[w];
-  const FdCell& cell = cells[row];
-  const float t = static_cast<float>(*time);
-  const int nr = cell.role == 2 ? 4 : (cell.role == 3 ? 6 : 0);
-  const bool own = cell.role == 1 && cell.kind != kPressureDirichlet;
-  float fu[7], fr[6];
+  {
+    static_assert(sizeof(FdCell) % 8 == 0, "copied in 8-byte words");
+    const unsigned long long* from = reinterpret_cast<const unsigned long long*>(cells + row);
+    unsigned long long* to = reinterpret_cast<unsigned long long*>(rec[threadIdx.x >> 5]);
+    for (int k = lane; k < static_cast<int>(sizeof(FdCell) / 8); k += 32) to[k] = from[k];
+    __syncwarp();
+  }
+  const FdCell& cell = *reinterpret_cast<const FdCell*>(rec[threadIdx.x >> 5]);
+  // ... and the prescribed velocities its reads name (before the ramp), a lane
+  // each: read where they are used, they were up to 13 memory latencies in a row
+  __shared__ float4 pres_s[kFdThreads / 32][13];
+  float4* pres = pres_s[threadIdx.x >> 5];
+  if (lane < 13) {
+    int from = -1;
+    if (lane < 7) {
+      if (cell.u[lane].code == kFdPrescribed) from = static_cast<int>(cell.u[lane].idx);
+    } else if (ROLE > 1 && lane - 7 < (ROLE == 2 ? 4 : 6)) {
+      const FdRRead& r = cell.r[lane - 7];
+      if (r.code == kFdRhoBmPre || r.code == kFdRhoBmNew) from = r.urow;
+    }
+    if (from >= 0) {
+      const FdCell& c = cells[from];
+      pres[lane] = make_float4(c.u_base[0], c.u_base[1], c.u_base[2], c.ramp_end);
+    }
+  }
+  __syncwarp();
+  pdl_wait();
+  const float t = static_cast<float>(*time + time_shift);
+  constexpr int nr = ROLE == 2 ? 4 : (ROLE == 3 ? 6 : 0);
+  const bool own = ROLE == 1 && cell.kind != kPressureDirichlet;
+  // Every value the warp sums, one population per lane: of each velocity read
+  // its density and momentum, of each density read (and a plane cell's own
+  // populations) the plain sum, or velocityBMRho's outgoing and wall sums.
+  constexpr int nv = 28 + 2 * nr + (ROLE == 1 ? 2 : 0);
+  float v[nv];
 #pragma unroll
   for (int j = 0; j < 7; ++j) {
     const FdURead& r = cell.u[j];
-    fu[j] = act && r.code == kFdFluid ? Store<T>::ld(state + i * qs + r.idx, inv_s) : 0.f;
+    v[4 * j] = act && r.code == kFdFluid ? Store<T>::ld(state + i * qs + r.idx, inv_s) : 0.f;
   }
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
+  for (int j = 0; j < nr; ++j) {
     const FdRRead& r = cell.r[j];
-    float v = 0.f;
-    if (act && j < nr && r.code != kFdRhoConst)
-      v = r.code == kFdRhoSumPre || r.code == kFdRhoBmPre ? Store<T>::ld(state + i * qs + r.idx, inv_s)
+    float x = 0.f;
+    if (act && r.code != kFdRhoConst)
+      x = r.code == kFdRhoSumPre || r.code == kFdRhoBmPre ? Store<T>::ld(state + i * qs + r.idx, inv_s)
                                                           : fnew[r.idx * kQ + i];
-    fr[j] = v;
+    v[28 + 2 * j] = x;
   }
-  const float fo = act && own ? Store<T>::ld(state + i * qs + cell.slot, inv_s) : 0.f;
+  if constexpr (ROLE == 1) v[28] = act && own ? Store<T>::ld(state + i * qs + cell.slot, inv_s) : 0.f;
+  const float shift = cr_shift ? *cr_shift : 0.f;
+#pragma unroll
+  for (int j = 0; j < 7; ++j)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) v[4 * j + 1 + a] = ci[a] * v[4 * j];
+  auto split = [&](int k, int d, int o) {  // velocityBMRho's sums of v[k]
+    const int c = d == 0 ? ci[0] : (d == 1 ? ci[1] : ci[2]);
+    const float x = v[k];
+    v[k] = c == o ? x : 0.f;
+    v[k + 1] = c == 0 ? x : 0.f;
+  };
+#pragma unroll
+  for (int j = 0; j < nr; ++j) {
+    const FdRRead& r = cell.r[j];
+    v[28 + 2 * j + 1] = 0.f;
+    if (r.code == kFdRhoBmPre || r.code == kFdRhoBmNew) split(28 + 2 * j, r.d, r.o);
+  }
+  if constexpr (ROLE == 1) split(28, cell.d, cell.o);
+  // All sums together, step by step of the butterfly: their shuffles are
+  // independent (one sum after the other left a warp waiting 5 shuffles per
+  // sum, 40 sums in a row: 7 us per launch).
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < nv; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
   // the seven velocities
   float uu[7][3];
 #pragma unroll
   for (int j = 0; j < 7; ++j) {
     const FdURead& r = cell.u[j];
-    if (r.code == kFdZero) {
-      uu[j][0] = uu[j][1] = uu[j][2] = 0.f;
-    } else if (r.code == kFdFluid) {
-      const float dh = warp_sum(fu[j]);
-      const float k = 1.f / (1.f + dh);
+    const float k = 1.f / (1.f + v[4 * j]);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) uu[j][a] = warp_sum(ci[a] * fu[j]) * k;
-    } else {
-      prescribed(cells, static_cast<int>(r.idx), t, uu[j]);
-    }
+    for (int a = 0; a < 3; ++a) uu[j][a] = r.code == kFdFluid ? v[4 * j + 1 + a] * k : 0.f;
+    if (r.code == kFdPrescribed) prescribed(pres[j], t, uu[j]);
 #pragma unroll
     for (int a = 0; a < 3; ++a)
       if (r.flip >> a & 1) uu[j][a] = -uu[j][a];
   }
-  // velocityBMRho of values v held one population per lane
-  auto bm = [&](float v, int d, int o, const float u[3]) {
-    const float out = warp_sum(ci[d] == o ? v : 0.f), wall = warp_sum(ci[d] == 0 ? v : 0.f);
-    return (2.f * out + wall + 1.f) / (1.f + o * u[d]);
+  auto bm = [&](int k, int d, int o, const float u[3]) {
+    const float ud = d == 0 ? u[0] : (d == 1 ? u[1] : u[2]);
+    return (2.f * v[k] + v[k + 1] + 1.f) / (1.f + o * ud);
   };
-  float rr[6];
+  float rr[nr > 0 ? nr : 1];
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    rr[j] = 0.f;
-    if (j >= nr) continue;
+  for (int j = 0; j < nr; ++j) {
     const FdRRead& r = cell.r[j];
     if (r.code == kFdRhoConst) {
       rr[j] = r.val;
@@ -184,33 +239,37 @@ k_fd_reconstruct(const T* state, long long qs, float inv_s, const FdCell* cells,
       // a kBulk cell's stored density under ConstRhoBGK carries the 1 -
       // average_rho its level's last collide added, if that collide came
       // after the level's stream (urow = 1 marks a kBulk cell)
-      const float shift = (r.code == kFdRhoSumPre && r.urow == 1 && cr_shift) ? *cr_shift : 0.f;
-      rr[j] = 1.f + warp_sum(fr[j]) - shift;
+      rr[j] = 1.f + v[28 + 2 * j] - (r.code == kFdRhoSumPre && r.urow == 1 ? shift : 0.f);
     } else {
       float u[3];
-      prescribed(cells, r.urow, t, u);
-      rr[j] = bm(fr[j], r.d, r.o, u);
+      prescribed(pres[7 + j], t, u);
+      rr[j] = bm(28 + 2 * j, r.d, r.o, u);
     }
   }
   float du[3][3];
   float rho;
-  if (cell.role == 1) {
+  if constexpr (ROLE == 1) {
     const int d = cell.d, o = cell.o;
-    rho = cell.kind == kPressureDirichlet ? cell.rho_target : bm(fo, d, o, uu[0]);
-    normal_grad(uu[0], uu[1], uu[2], o, du[d]);
-    const int t0 = (d + 1) % 3 < (d + 2) % 3 ? (d + 1) % 3 : (d + 2) % 3;
-    const int t1 = 3 - d - t0;
+    rho = cell.kind == kPressureDirichlet ? cell.rho_target : bm(28, d, o, uu[0]);
+    float gn[3];
+    normal_grad(uu[0], uu[1], uu[2], o, gn);
+    const int t0 = d == 0 ? 1 : 0;  // the lower of the two tangential axes
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      du[t0][b] = (uu[3][b] - uu[4][b]) * 0.5f;
-      du[t1][b] = (uu[5][b] - uu[6][b]) * 0.5f;
-    }
-  } else if (cell.role == 2) {
-    const int p = cell.ax[0], d1 = cell.ax[1], d2 = cell.ax[2];
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) du[p][b] = (uu[1][b] - uu[2][b]) * 0.5f;
-    normal_grad(uu[0], uu[3], uu[4], cell.nrm[0], du[d1]);
-    normal_grad(uu[0], uu[5], uu[6], cell.nrm[1], du[d2]);
+      for (int b = 0; b < 3; ++b)
+        du[a][b] = a == d ? gn[b] : (a == t0 ? (uu[3][b] - uu[4][b]) * 0.5f : (uu[5][b] - uu[6][b]) * 0.5f);
+  } else if constexpr (ROLE == 2) {
+    const int p = cell.ax[0], d1 = cell.ax[1];
+    float gp[3], g1[3], g2[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) gp[b] = (uu[1][b] - uu[2][b]) * 0.5f;
+    normal_grad(uu[0], uu[3], uu[4], cell.nrm[0], g1);
+    normal_grad(uu[0], uu[5], uu[6], cell.nrm[1], g2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) du[a][b] = a == p ? gp[b] : (a == d1 ? g1[b] : g2[b]);
     rho = 2.f / 3.f * (rr[0] + rr[1]) - 1.f / 6.f * (rr[2] + rr[3]);
   } else {
 #pragma unroll
@@ -248,20 +307,39 @@ k_fd_reconstruct(const T* state, long long qs, float inv_s, const FdCell* cells,
 // corners; bounce-back cells the full-way swap of their streamed state (kept
 // in their row); pressure cells unchanged.  Source: the rows (the last
 // pass's, or the initial state's), or the state itself when fnew is null.
+//
+// ConstRhoBGK: each CTA's sum of the velocity cells' collide densities goes to
+// up.bpart, and the last CTA to finish forms the average the step's collide
+// uses (k_cr_update's sums in its order: 256 strided sums, then the shuffle
+// trees), which saves that launch.
+struct FdCrUpdate {
+  double* bpart;              // null: no statistics
+  unsigned int* done;
+  double* avg;
+  const double* part;
+  int nparts;
+  long long count, bcount;
+  float* shift;
+};
 template <typename T>
 __global__ void __launch_bounds__(kFdThreads)
 k_fd_collide(T* state, long long qs, float scale, float inv_s, const FdCell* cells, int n, float* fnew,
-             const double* time, double time_shift, float omega, double* cr_part) {
+             const double* time, double time_shift, float omega, const FdCrUpdate up) {
+  pdl_trigger();
   const int row = blockIdx.x * kFdThreads + threadIdx.x;
+  const FdCell& cell = cells[row < n ? row : 0];
+  const int role = cell.role, kind = cell.kind, cd = cell.d, co = cell.o;
+  const long long slot = cell.slot;
+  const float ub[3] = {cell.u_base[0], cell.u_base[1], cell.u_base[2]}, ramp_end = cell.ramp_end;
+  pdl_wait();
   double stat = 0.0;  // ConstRhoBGK statistics: the velocity cell's collide density
   if (row < n) {
-  const FdCell& cell = cells[row];
   float f[kQ];
-  if (cell.role == 0) {
+  if (role == 0) {
     // a bounce-back cell (the dispatcher's kBounceBack arm, bc_dispatcher.h:
     // 55-67): its streamed populations are its row (the state after the
     // step), then the full-way swap f_i <- f_opp(i)
-    load_pops(state, qs, cell.slot, inv_s, f);
+    load_pops(state, qs, slot, inv_s, f);
     float g[kQ];
 #pragma unroll
     for (int i = 0; i < kQ; ++i) {
@@ -274,48 +352,85 @@ k_fd_collide(T* state, long long qs, float scale, float inv_s, const FdCell* cel
 #pragma unroll
     for (int i = 0; i < kQ; ++i) f[i] = fnew[static_cast<long long>(row) * kQ + i];
   } else {
-    load_pops(state, qs, cell.slot, inv_s, f);
+    load_pops(state, qs, slot, inv_s, f);
   }
-  if (cell.kind == kVelocityDirichlet) {
-    float u[3];
-    prescribed(cells, row, static_cast<float>(*time + time_shift), u);
-    const float rho = cell.role == 1 ? bm_rho(f, cell.d, cell.o, u) : 1.f + sum_pops(f);
+  if (kind == kVelocityDirichlet) {
+    const float r = ramp(static_cast<float>(*time + time_shift), ramp_end);
+    const float u[3] = {r * ub[0], r * ub[1], r * ub[2]};
+    const float rho = role == 1 ? bm_rho(f, cd, co, u) : 1.f + sum_pops(f);
     stat = rho;
     const float usq = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
 #pragma unroll
     for (int i = 0; i < kQ; ++i) f[i] = f[i] * (1.f - omega) + omega * feq_i(i, rho, u, usq);
   }
 #pragma unroll
-  for (int i = 0; i < kQ; ++i) Store<T>::st(state + i * qs + cell.slot, f[i], scale);
+  for (int i = 0; i < kQ; ++i) Store<T>::st(state + i * qs + slot, f[i], scale);
   }
-  if (cr_part) {  // this CTA's sum, in a fixed order
-    for (int o = 16; o > 0; o >>= 1) stat += __shfl_down_sync(0xffffffffu, stat, o);
-    __shared__ double ws[kFdThreads / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = stat;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double sum = 0.0;
-      for (int w = 0; w < kFdThreads / 32; ++w) sum += ws[w];
-      cr_part[blockIdx.x] = sum;
+  if (!up.bpart) return;
+  // this CTA's sum, in a fixed order
+  for (int o = 16; o > 0; o >>= 1) stat += __shfl_down_sync(0xffffffffu, stat, o);
+  __shared__ double ws[kThreads / 32][2];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0) ws[warp][0] = stat;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double sum = 0.0;
+    for (int w = 0; w < kFdThreads / 32; ++w) sum += ws[w][0];
+    up.bpart[blockIdx.x] = sum;
+    __threadfence();
+    last = atomicInc(up.done, gridDim.x - 1) == gridDim.x - 1;  // wraps to 0 for the next launch
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  for (int h = 0; h < kThreads / kFdThreads; ++h) {  // k_cr_update's thread h * kFdThreads + threadIdx.x
+    double v[2] = {0.0, 0.0};
+    for (int p = h * kFdThreads + threadIdx.x; p < up.nparts; p += kThreads) v[0] += __ldcg(up.part + p);
+    for (int p = h * kFdThreads + threadIdx.x; p < static_cast<int>(gridDim.x); p += kThreads) v[1] += __ldcg(up.bpart + p);
+    for (int k = 0; k < 2; ++k) {
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+      if (lane == 0) ws[h * (kFdThreads / 32) + warp][k] = v[k];
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+    double v[2];
+    for (int k = 0; k < 2; ++k) {
+      v[k] = lane < kThreads / 32 ? ws[lane][k] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+    }
+    if (lane == 0) {
+      cr_average(up.avg, v[0], up.count, v[1], up.bcount);
+      if (up.shift) *up.shift = static_cast<float>(1.0 - *up.avg);
     }
   }
 }
 
-__global__ void k_fd_tick(double* time) { *time += 1.0; }
+__global__ void k_fd_tick(double* time) {
+  pdl_wait();
+  *time += 1.0;
+}
 
 // The pass's rewritten rows into the state (velocity and pressure cells; the
 // bounce-back cells keep their streamed populations until their collide).
 template <typename T>
 __global__ void __launch_bounds__(kFdThreads)
-k_fd_store(T* state, long long qs, float scale, const FdCell* cells, int n, const float* fnew, double* tick) {
+k_fd_store(T* state, long long qs, float scale, const FdCell* cells, int n, const float* fnew, double* tick, double ticks) {
+  pdl_trigger();
   const int row = blockIdx.x * kFdThreads + threadIdx.x;
+  const int role = row < n ? cells[row].role : 0;
+  const long long slot = row < n ? cells[row].slot : 0;
+  pdl_wait();
   // the boundary clock's tick, where this is the step's last pass (no kernel
   // of the pass reads the clock after the reconstruction)
-  if (tick && row == 0) *tick += 1.0;
-  if (row >= n || cells[row].role == 0) return;
+  if (tick && row == 0) *tick += ticks;
+  if (role == 0) return;
+  float f[kQ];  // loads before stores (they may alias for all the compiler knows)
 #pragma unroll
-  for (int i = 0; i < kQ; ++i)
-    Store<T>::st(state + i * qs + cells[row].slot, fnew[static_cast<long long>(row) * kQ + i], scale);
+  for (int i = 0; i < kQ; ++i) f[i] = fnew[static_cast<long long>(row) * kQ + i];
+#pragma unroll
+  for (int i = 0; i < kQ; ++i) Store<T>::st(state + i * qs + slot, f[i], scale);
 }
 
 // The Dirichlet cells' populations before their collide (the initial state)
@@ -366,23 +481,26 @@ namespace {
 
 template <typename T>
 cudaError_t launch_fd_reconstruct(const void* state, long long qs, float inv_s, const FdCell* cells, const int* list,
-                                  int n, float* fnew, const double* time, float omega, const float* cr_shift,
-                                  cudaStream_t s) {
+                                  int role, int n, float* fnew, const double* time, double time_shift, float omega,
+                                  const float* cr_shift, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const unsigned grid = static_cast<unsigned>((static_cast<long long>(n) * 32 + kFdThreads - 1) / kFdThreads);
-  k_fd_reconstruct<T><<<grid, kFdThreads, 0, s>>>(static_cast<const T*>(state), qs, inv_s, cells, list, n, fnew,
-                                                  time, omega, cr_shift);
-  return cudaGetLastError();
+  auto* k = role == 1 ? k_fd_reconstruct<T, 1> : (role == 2 ? k_fd_reconstruct<T, 2> : k_fd_reconstruct<T, 3>);
+  const cudaError_t e = launch_chain(k, dim3(grid), dim3(kFdThreads), 0, s, static_cast<const T*>(state), qs, inv_s, cells,
+                                     list, n, fnew, time, time_shift, omega, cr_shift);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_fd_collide(void* state, long long qs, float scale, float inv_s, const FdCell* cells, int n,
-                              float* fnew, const double* time, double time_shift, float omega, double* cr_part,
-                              cudaStream_t s) {
+                              float* fnew, const double* time, double time_shift, float omega, double* bpart,
+                              unsigned int* done, double* avg, const double* part, int nparts, long long count,
+                              long long bcount, float* shift, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  k_fd_collide<T><<<fd_grid(n), kFdThreads, 0, s>>>(static_cast<T*>(state), qs, scale, inv_s, cells, n, fnew, time,
-                                                     time_shift, omega, cr_part);
-  return cudaGetLastError();
+  const FdCrUpdate up{bpart, done, avg, part, nparts, count, bcount, shift};
+  const cudaError_t e = launch_chain(k_fd_collide<T>, dim3(fd_grid(n)), dim3(kFdThreads), 0, s, static_cast<T*>(state), qs,
+                                     scale, inv_s, cells, n, fnew, time, time_shift, omega, up);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <typename T>
@@ -402,26 +520,28 @@ cudaError_t launch_fd_fields(const FdCell* cells, int n, const float* fnew, cons
 
 template <typename T>
 cudaError_t launch_fd_store(void* state, long long qs, float scale, const FdCell* cells, int n, const float* fnew,
-                            double* tick, cudaStream_t s) {
+                            double* tick, double ticks, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  k_fd_store<T><<<fd_grid(n), kFdThreads, 0, s>>>(static_cast<T*>(state), qs, scale, cells, n, fnew, tick);
-  return cudaGetLastError();
+  const cudaError_t e = launch_chain(k_fd_store<T>, dim3(fd_grid(n)), dim3(kFdThreads), 0, s, static_cast<T*>(state), qs,
+                                     scale, cells, n, fnew, tick, ticks);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 template cudaError_t launch_fd_store<float>(void*, long long, float, const FdCell*, int, const float*, double*,
-                                           cudaStream_t);
+                                           double, cudaStream_t);
 template cudaError_t launch_fd_store<__half>(void*, long long, float, const FdCell*, int, const float*, double*,
-                                            cudaStream_t);
+                                            double, cudaStream_t);
 
 cudaError_t launch_fd_tick(double* time, cudaStream_t s) {
-  k_fd_tick<<<1, 1, 0, s>>>(time);
-  return cudaGetLastError();
+  const cudaError_t e = launch_chain(k_fd_tick, dim3(1), dim3(1), 0, s, time);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 #define OCTLB_FD_INST(T)                                                                                      \
-  template cudaError_t launch_fd_reconstruct<T>(const void*, long long, float, const FdCell*, const int*, int, \
-                                                float*, const double*, float, const float*, cudaStream_t);  \
+  template cudaError_t launch_fd_reconstruct<T>(const void*, long long, float, const FdCell*, const int*, int, int, \
+                                                float*, const double*, double, float, const float*, cudaStream_t);          \
   template cudaError_t launch_fd_collide<T>(void*, long long, float, float, const FdCell*, int, float*,        \
-                                            const double*, double, float, double*, cudaStream_t);
+                                            const double*, double, float, double*, unsigned int*, double*,     \
+                                            const double*, int, long long, long long, float*, cudaStream_t);
 template cudaError_t launch_fd_rows_from_state<float>(const void*, long long, float, const FdCell*, int, float*,
                                                      cudaStream_t);
 template cudaError_t launch_fd_rows_from_state<__half>(const void*, long long, float, const FdCell*, int, float*,

@@ -948,10 +948,7 @@ k_cr_update(double* avg, const double* part, int nparts, long long count, const 
   for (int p = threadIdx.x; p < nbparts; p += kThreads) v[1] += bpart[p];
   block_reduce<2>(v);
   if (threadIdx.x == 0) {
-    if (bcount == 0)
-      *avg = count > 0 ? (2.0 - *avg) + v[0] / static_cast<double>(count) : 1.0;
-    else
-      *avg = (v[0] + static_cast<double>(count) * (2.0 - *avg) + v[1]) / static_cast<double>(count + bcount);
+    cr_average(avg, v[0], count, v[1], bcount);
     if (shift) *shift = static_cast<float>(1.0 - *avg);
   }
 }

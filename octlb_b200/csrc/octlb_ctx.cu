@@ -161,16 +161,18 @@ int launch_level_step(octlb_ctx* ctx, Level& L) {
   } else if (ctx->const_rho) {
     // ConstRhoBGK: average_rho from the last collide's statistics
     // (time_loop.h:220-222), then the step whose collide uses it
-    CK(launch_cr_update(ctx->cr_avg.as<double>(), ctx->cr_part.as<double>(), ctx->cr_nparts + ctx->cr_pparts,
-                        ctx->cr_count, ctx->fd_cr_part.as<double>(), ctx->fd_cr_parts, ctx->fd_vel,
-                        ctx->cr_shift.as<float>() + L.lvl, ctx->stream));
+    if (!fd_updates_average(ctx, L)) {
+      CK(launch_cr_update(ctx->cr_avg.as<double>(), ctx->cr_part.as<double>(), ctx->cr_nparts + ctx->cr_pparts,
+                          ctx->cr_count, ctx->fd_cr_part.as<double>(), ctx->fd_cr_parts, ctx->fd_vel,
+                          ctx->cr_shift.as<float>() + L.lvl, ctx->stream));
+      ++ctx->launch_count;
+    }
     const bool links = ctx->stream_mode == OCTLB_STREAM_LINKS;
     if (L.use_map) {
       CK(launch_step_map<T>(a, L.near, links, L.has_flags, kCollConstRho, ctx->stream));
-      ++ctx->launch_count;
     } else {
       CK(launch_step_cr<T>(a, L.near, links, L.has_flags, ctx->stream));
-      ctx->launch_count += 1 + (L.near.n > 0 ? 1 : 0);
+      if (L.near.n > 0) ++ctx->launch_count;
     }
   } else if (L.aa) {
     // AA order: cur is the layout (1: reversed), both buffers the same memory
@@ -1526,7 +1528,13 @@ int advance_graph(octlb_ctx* ctx, int count) {
     const std::vector<int> c0 = ctx->counters_collide;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     int rc = OCTLB_OK;
-    for (int k = 0; k < count && rc == OCTLB_OK; ++k) rc = advance_one_launches<T>(ctx);
+    ctx->batch_len = count;
+    for (int k = 0; k < count && rc == OCTLB_OK; ++k) {
+      ctx->batch_pos = k;
+      rc = advance_one_launches<T>(ctx);
+    }
+    ctx->batch_pos = 0;
+    ctx->batch_len = 1;
     cudaGraph_t g = nullptr;
     const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }

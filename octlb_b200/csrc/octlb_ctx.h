@@ -344,6 +344,7 @@ struct octlb_ctx {
     std::vector<int> dcollide;
   };
   std::map<std::pair<uint64_t, int>, GraphEntry> graphs;
+  int batch_pos = 0, batch_len = 1; // the advance_one being issued within its graph, and the graph's
   bool use_graphs = true;           // OCTLB_NO_GRAPH=1 launches kernel by kernel
   bool use_pdl = true;              // OCTLB_NO_PDL=1: plain stream order between the step's kernels
   float prolong_scale = 0.f, restrict_scale = 0.f;
@@ -386,7 +387,7 @@ struct octlb_ctx {
   // ConstRhoBGK with the pass: per-CTA sums of the velocity cells' collide
   // densities (the boundary part of the statistics), over fd_vel cells
   bool fd_single = false;           // the pass on one level: its store ticks the clock
-  DevBuf fd_cr_part;
+  DevBuf fd_cr_part, fd_done;       // ... and the collide's count of finished CTAs
   // ConstRhoBGK: per level the density shift 1 - average_rho its kBulk
   // cells' stored state carries (0 after a stream-only step), which the
   // finite-difference pass removes from the densities it reads
@@ -425,6 +426,7 @@ int comm_nranks(const octlb_comm* comm);
 template <typename T> int fd_after_step(octlb_ctx* ctx, Level& L);
 template <typename T> int fd_before_step(octlb_ctx* ctx, Level& L);
 int fd_end_of_step(octlb_ctx* ctx);
+bool fd_updates_average(const octlb_ctx* ctx, const Level& L);
 int fd_fix_fields(octlb_ctx* ctx, Level& L, const int* gid, double* rho, double* u);
 void clear_graphs(octlb_ctx* ctx);
 void comm_detach(octlb_ctx* ctx);

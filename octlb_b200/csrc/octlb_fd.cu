@@ -17,18 +17,19 @@
 
 namespace octlb_gpu {
 template <typename T>
-cudaError_t launch_fd_reconstruct(const void*, long long, float, const FdCell*, const int*, int, float*,
-                                  const double*, float, const float*, cudaStream_t);
+cudaError_t launch_fd_reconstruct(const void*, long long, float, const FdCell*, const int*, int, int, float*, const double*,
+                                  double, float, const float*, cudaStream_t);
 template <typename T>
-cudaError_t launch_fd_collide(void*, long long, float, float, const FdCell*, int, float*, const double*,
-                              double, float, double*, cudaStream_t);
+cudaError_t launch_fd_collide(void*, long long, float, float, const FdCell*, int, float*, const double*, double, float,
+                              double*, unsigned int*, double*, const double*, int, long long, long long, float*,
+                              cudaStream_t);
 unsigned fd_collide_parts(int n);
 cudaError_t launch_fd_tick(double*, cudaStream_t);
 template <typename T>
 cudaError_t launch_fd_rows_from_state(const void*, long long, float, const FdCell*, int, float*, cudaStream_t);
 cudaError_t launch_fd_fields(const FdCell*, int, const float*, const int*, FastDiv, double*, double*, cudaStream_t);
 template <typename T>
-cudaError_t launch_fd_store(void*, long long, float, const FdCell*, int, const float*, double*, cudaStream_t);
+cudaError_t launch_fd_store(void*, long long, float, const FdCell*, int, const float*, double*, double, cudaStream_t);
 }  // namespace octlb_gpu
 
 using namespace octlb_gpu;
@@ -155,6 +156,10 @@ namespace octlb_host {
 // planes, edges, corners into the rows, then the rows into the state,
 // uncollided, as the reference rewrites the cells in place -- a later pass
 // on a level that has not stepped since reads them as its "pre" values.
+// The boundary clock of the current step: steps of one graph behind the first
+// count from the clock at its start (single-level meshes; others tick per step).
+double fd_shift(const octlb_ctx* ctx) { return ctx->fd_single ? ctx->batch_pos : 0.0; }
+
 template <typename T>
 int fd_after_step(octlb_ctx* ctx, Level& S) {
   (void)S;
@@ -169,33 +174,44 @@ int fd_after_step(octlb_ctx* ctx, Level& S) {
     for (int role = 1; role <= 3; ++role) {
       const int n = L.fd_count[role];
       if (n == 0) continue;
-      CK(launch_fd_reconstruct<T>(state, L.nslots, L.inv_scale, cells, L.fd_lists.as<int>() + L.fd_first[role], n,
-                                  fnew, time, omega, ctx->const_rho ? ctx->cr_shift.as<float>() + L.lvl : nullptr,
-                                  ctx->stream));
+      CK(launch_fd_reconstruct<T>(state, L.nslots, L.inv_scale, cells, L.fd_lists.as<int>() + L.fd_first[role], role,
+                                  n, fnew, time, fd_shift(ctx), omega,
+                                  ctx->const_rho ? ctx->cr_shift.as<float>() + L.lvl : nullptr, ctx->stream));
       ++ctx->launch_count;
     }
-    // on a single-level mesh this is the step's only pass: the store ticks
-    // the boundary clock in place of a launch of its own
+    // On a single-level mesh this is the step's only pass.  A step that another
+    // of its graph follows needs no store: the next collide takes the rows and
+    // writes every one of these cells.  The last one's store also ticks the
+    // boundary clock for all of them.
+    if (ctx->fd_single && ctx->batch_pos + 1 < ctx->batch_len) continue;
     CK(launch_fd_store<T>(state, L.nslots, L.scale, cells, L.fd_rows, fnew,
-                          ctx->fd_single ? ctx->fd_time.as<double>() : nullptr, ctx->stream));
+                          ctx->fd_single ? ctx->fd_time.as<double>() : nullptr, ctx->batch_len, ctx->stream));
     ++ctx->launch_count;
   }
   return OCTLB_OK;
+}
+
+// Whether the boundary cells' collide of level L forms ConstRhoBGK's average
+// (its last CTA, in place of the update's own launch).
+bool fd_updates_average(const octlb_ctx* ctx, const Level& L) {
+  return ctx->fd_on && ctx->const_rho && L.lvl == ctx->cr_level && L.nblk > 0 && L.fd_rows > 0;
 }
 
 // The collide of level L's boundary cells at the start of its step
 // (collide_level's per-cell dispatch, domain_boundary_handler.cpp:60-79), at
 // this advance_one's time, from the rows the last pass left.  Under
 // ConstRhoBGK the velocity cells' collide densities go to the partials the
-// average update then reads.
+// average update then reads, and the last CTA makes that update.
 template <typename T>
 int fd_before_step(octlb_ctx* ctx, Level& L) {
   if (!ctx->fd_on || L.nblk == 0 || L.fd_rows == 0) return OCTLB_OK;
   CK(launch_fd_collide<T>(cur_buf(L), L.nslots, L.scale, L.inv_scale, L.fd_cells.as<FdCell>(), L.fd_rows,
-                          L.fd_new.as<float>(), ctx->fd_time.as<double>(), 0.0,
+                          L.fd_new.as<float>(), ctx->fd_time.as<double>(), fd_shift(ctx),
                           static_cast<float>(ctx->omega_l[L.lvl]),
-                          ctx->const_rho && L.lvl == ctx->cr_level ? ctx->fd_cr_part.as<double>() : nullptr,
-                          ctx->stream));
+                          fd_updates_average(ctx, L) ? ctx->fd_cr_part.as<double>() : nullptr,
+                          ctx->fd_done.as<unsigned int>(), ctx->cr_avg.as<double>(), ctx->cr_part.as<double>(),
+                          ctx->cr_nparts + ctx->cr_pparts, ctx->cr_count, ctx->fd_vel,
+                          ctx->const_rho ? ctx->cr_shift.as<float>() + L.lvl : nullptr, ctx->stream));
   ++ctx->launch_count;
   return OCTLB_OK;
 }
@@ -504,6 +520,7 @@ int octlb_gpu_set_fd_boundary_inlets(octlb_ctx* ctx, const int types[6], const d
   for (const auto& c : cells) total += c.size();
   if (total == 0) return fail(ctx, OCTLB_EINVAL, "fd boundary: no Dirichlet or bounce-back cells");
   CK(upload(ctx->fd_time, std::vector<double>{0.0}));
+  CK(ctx->fd_done.alloc(sizeof(unsigned int)));
   // ConstRhoBGK (chosen before): the finest level's velocity cells'
   // collide densities join its statistics (the reference's
   // kFluidAndBoundary scope, collected where level >= max_level_,
