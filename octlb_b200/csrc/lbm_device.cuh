@@ -92,23 +92,17 @@ __device__ __forceinline__ float pull_value(const StepArgs& a, const T* src, int
   return Store<T>::ld(src + i * a.qs + s, a.inv_scale);
 }
 
-// Halo item k of an open block (block_lattice.h:70-89): item (page, block,
-// halo index, population i); the page slot it writes, and the slot its torus
-// pull reads (own core, the neighbour core the exchange copies, or the own
-// halo page).
-__device__ __forceinline__ void rotate_slots(const StepArgs& a, uint32_t k, long long& dst, long long& src, int& i) {
-  const int4 it = reinterpret_cast<const int4*>(a.open_pages)[k];
-  i = it.w;
-  const int cells = a.np * a.np * a.np;
-  int sp = a.hpos[it.z] - a.off_pad[i];
-  sp = sp < 0 ? sp + cells : (sp >= cells ? sp - cells : sp);
-  const int X = static_cast<int>(a.div_np2.div(static_cast<uint32_t>(sp)));
-  const int rem = sp - X * a.np * a.np;
-  const int Y = static_cast<int>(a.div_np.div(static_cast<uint32_t>(rem)));
-  const int Z = rem - Y * a.np;
-  bool halo;
-  src = resolve(a, static_cast<uint32_t>(it.y), X, Y, Z, halo);
-  dst = a.halo_base + static_cast<long long>(it.x) * a.n_halo + it.z;
+// Halo item k of an open block (block_lattice.h:70-89), resolved on the host:
+// the page slot it writes, the slot its torus pull reads (own core, the
+// neighbour core the exchange copies, or the own halo page), its population,
+// and whether that source is a tree-boundary fill.  (Resolved here, an item was
+// a chain of five dependent reads: halo index, position, base or page, value.)
+__device__ __forceinline__ bool rotate_slots(const StepArgs& a, uint32_t k, long long& dst, long long& src, int& i) {
+  const int4 it = __ldg(reinterpret_cast<const int4*>(a.open_items) + k);
+  dst = it.x;
+  src = it.y;
+  i = it.z;
+  return it.w != 0;
 }
 
 // Lane-parallel forms (lane i < 19 holds population i): lattice vectors and

@@ -149,7 +149,6 @@ __global__ void __launch_bounds__(THREADS, WARPS * 32 / THREADS) k_step_map(cons
   }
   const uint32_t bid = blockIdx.x - near_ctas;
   if (bid >= core_ctas) {
-    pdl_wait();
     rotate_item<T>(a, (bid - core_ctas) * THREADS + tid);
     return;
   }

@@ -27,13 +27,12 @@ __device__ __forceinline__ void rotate_item(const StepArgs& a, uint32_t k) {
   if (k >= static_cast<uint32_t>(a.n_open)) return;
   long long d, sl;
   int i;
-  rotate_slots(a, k, d, sl, i);
+  const bool fill = rotate_slots(a, k, d, sl, i);
+  pdl_wait();
   const T* src = static_cast<const T*>(a.src);
   T* dst = static_cast<T*>(a.dst);
-  if (sl >= a.halo_base && a.fill_of && a.fill_of[(sl - a.halo_base) * kQ + i] >= 0)
-    Store<T>::st(dst + i * a.qs + d, pull_value(a, src, i, sl), a.scale);  // source is a boundary fill
-  else
-    dst[i * a.qs + d] = src[i * a.qs + sl];
+  if (fill) Store<T>::st(dst + i * a.qs + d, pull_value(a, src, i, sl), a.scale);
+  else dst[i * a.qs + d] = src[i * a.qs + sl];
 }
 
 // Cells flagged kFlagNear (links stream rule): the per-cell link rule of

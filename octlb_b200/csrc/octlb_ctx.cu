@@ -869,7 +869,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
         if (open) needs_page[lb] = 1;
       }
     }
-    std::vector<int> page_of(static_cast<size_t>(L.nblk), -1), open_pages;
+    std::vector<int> page_of(static_cast<size_t>(L.nblk), -1);
     for (int lb = 0; lb < L.nblk; ++lb)
       if (needs_page[lb]) page_of[lb] = L.n_pages++;
     // Torus-streamed halo populations of open blocks: the (slot, population)
@@ -918,7 +918,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
         }
       }
     }
-    open_pages = halo_items;
     L.n_open = static_cast<int>(halo_items.size() / 4);
     L.n_halo = L.n_pages > 0 ? H : 0;
     // even slot count: population rows start on 2-element boundaries
@@ -962,6 +961,21 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
       if (page_of[lb] >= 0) return core_end + static_cast<long long>(page_of[lb]) * H + hmap[P];
       return -1;
     };
+    // The halo items resolved: page slot written, slot its torus pull reads
+    // (block_lattice.h:70-89), population, 1 where that source is a fill.
+    std::vector<int> open_items;
+    open_items.reserve(halo_items.size());
+    for (size_t k = 0; k < halo_items.size(); k += 4) {
+      const int lb = halo_items[k + 1], hidx = halo_items[k + 2], pop = halo_items[k + 3];
+      int sp = hpos[hidx] - (cx(pop) * np * np + cy(pop) * np + cz(pop));
+      sp = ((sp % np3) + np3) % np3;
+      const long long to = core_end + static_cast<long long>(halo_items[k]) * H + hidx;
+      const long long from = resolve_slot(lb, sp / (np * np), (sp / np) % np, sp % np);
+      if (from < 0 || from >= L.nslots || to >= L.nslots || L.nslots > INT_MAX)
+        return fail(ctx, OCTLB_EINVAL, "internal: halo item without a source");
+      const bool fill = from >= core_end && fill_of_h[static_cast<size_t>(from - core_end) * kQ + pop] >= 0;
+      open_items.insert(open_items.end(), {static_cast<int>(to), static_cast<int>(from), pop, fill ? 1 : 0});
+    }
     std::vector<int> slot_map;
     std::vector<float> wall_add, wall_dadd;  // per moving-wall position: the 19 wall terms, their velocity derivative
     if (map_step_eligible(n, L.nslots) && !(ctx->periodic && !L.has_flags)) {
@@ -1120,9 +1134,8 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
           return fail(ctx, OCTLB_EINVAL, "internal: boundary fill out of range");
       for (int v : lidx) if (v < -1 || v >= L.n_links) return fail(ctx, OCTLB_EINVAL, "internal: link index");
       for (int v : sidx) if (v < -1 || v >= L.n_save) return fail(ctx, OCTLB_EINVAL, "internal: save index");
-      for (size_t k = 0; k < open_pages.size(); k += 4)
-        if (!in(open_pages[k], L.n_pages) || !in(open_pages[k + 1], L.nblk) || !in(open_pages[k + 2], H) ||
-            !in(open_pages[k + 3], kQ))
+      for (size_t k = 0; k < open_items.size(); k += 4)
+        if (!in(open_items[k], ns) || open_items[k] < core_end || !in(open_items[k + 1], ns) || !in(open_items[k + 2], kQ))
           return fail(ctx, OCTLB_EINVAL, "internal: halo item");
       for (int lb = 0; lb < L.nblk; ++lb)
         for (int d = 0; d < 27; ++d) {
@@ -1174,7 +1187,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     CK(upload(L.hmap, hmap));
     CK(upload(L.blk_gid, std::vector<int>(L.blocks.begin(), L.blocks.begin() + L.nblk)));
     CK(upload(L.hpos, hpos));
-    CK(upload(L.open_pages, open_pages));
+    CK(upload(L.open_items, open_items));
     CK(upload(L.near_cells, near_cells));
     CK(upload(L.near_mask, nmask));
     CK(upload(L.near_slot, nslot));
@@ -1213,7 +1226,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     A.page_of = L.page_of.as<int>();
     A.hmap = L.hmap.as<int>();
     A.hpos = L.hpos.as<int>();
-    A.open_pages = L.open_pages.as<int>();
+    A.open_items = L.open_items.as<int>();
     A.n_open = L.n_open;
     A.n_halo = L.n_halo;
     A.nblk = L.nblk; A.n = n; A.np = np;

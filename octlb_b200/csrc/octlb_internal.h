@@ -33,7 +33,7 @@ struct StepArgs {
   const int* page_of;       // [nblk] halo page or -1
   const int* hmap;          // [(n+2)^3] padded position -> halo index (-1 in the core)
   const int* hpos;          // [n_halo] halo index -> padded linear position
-  const int* open_pages;    // [n_open][4] torus-streamed halo items: page, block, halo index, population
+  const int* open_items;    // [n_open][4] torus-streamed halo items: slot written, slot read, population, 1: a fill is read
   const int* slot_map;      // [nblk][(n+2)^3] slot of every padded position (k_step_map levels)
   const int* row_map;       // [nblk][3][(n+2)^2] slot map at Z = 1, 0 and n + 1 (kBlkRows blocks)
   const int* fill_of;       // [n_pages * n_halo][19] boundary fill writing (page slot, population), or -1
