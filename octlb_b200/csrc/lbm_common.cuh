@@ -87,6 +87,10 @@ struct FastDiv {
 // a predecessor writes.  A no-op for a kernel launched without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The dependents may be launched once every CTA has come here (they wait for
+// this grid's end before they read what it writes).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename T> struct Store;
 template <> struct Store<float> {
   __device__ static inline float ld(const float* p, float) { return *p; }

@@ -39,10 +39,6 @@ namespace {
 
 constexpr int kFdThreads = 128;
 
-// The dependents may be launched (they wait for this grid's end before they
-// read what it writes).
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // PolynomialStartScale: 10 x^3 - 15 x^4 + 6 x^5, x = t / t_end clamped to [0, 1].
 __device__ __forceinline__ float ramp(float t, float t_end) {
   if (t_end <= 0.f) return 1.f;

@@ -599,10 +599,12 @@ __device__ __forceinline__ void restrict_warp(const RestrictOp& op, int w, int l
 // warp per item, each on its own range of CTAs.  Operations that nothing
 // between them orders (a restriction into level l and the full-time
 // prolongation into level l with disjoint targets; two restrictions) share a
-// launch this way.
+// launch this way.  trigger: the next launch may start beside this one (its
+// CTAs read their tables while this one's finish; couple_triggers).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_couple(const ProlongOp p, const RestrictOp r0, const RestrictOp r1) {
+__global__ void __launch_bounds__(kThreads) k_couple(const ProlongOp p, const RestrictOp r0, const RestrictOp r1, int trigger) {
   __shared__ float fneq_s[kThreads / 32][kQ][kQ + 1];  // restriction: [warp][row][population]
+  if (trigger) pdl_trigger();
   const uint32_t gp = (static_cast<uint32_t>(p.n) * 32 + kThreads - 1) / kThreads;
   const uint32_t g0 = (static_cast<uint32_t>(r0.n) * 32 + kThreads - 1) / kThreads;
   const int lane = threadIdx.x & 31;
@@ -1078,11 +1080,11 @@ cudaError_t launch_add_force(const StepArgs& a, T* pops, const float* force, cud
 
 
 template <typename T>
-cudaError_t launch_couple(const ProlongOp& p, const RestrictOp& r0, const RestrictOp& r1, cudaStream_t s) {
+cudaError_t launch_couple(const ProlongOp& p, const RestrictOp& r0, const RestrictOp& r1, bool trigger, cudaStream_t s) {
   const uint32_t g = grid_for(static_cast<uint32_t>(p.n) * 32) + grid_for(static_cast<uint32_t>(r0.n) * 32) +
                      grid_for(static_cast<uint32_t>(r1.n) * 32);
   if (g == 0) return cudaSuccess;
-  const cudaError_t e = launch_chain(k_couple<T>, dim3(g), dim3(kThreads), 0, s, p, r0, r1);
+  const cudaError_t e = launch_chain(k_couple<T>, dim3(g), dim3(kThreads), 0, s, p, r0, r1, trigger ? 1 : 0);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 
@@ -1186,7 +1188,7 @@ cudaError_t launch_cr_update(double* avg, const double* part, int nparts, long l
   template cudaError_t launch_step_near<T>(const StepArgs&, const NearTables&, cudaStream_t);       \
   template cudaError_t launch_add_force<T>(const StepArgs&, T*, const float*, cudaStream_t);         \
   template cudaError_t launch_couple<T>(const ProlongOp&, const RestrictOp&, const RestrictOp&,    \
-                                        cudaStream_t);                                             \
+                                        bool, cudaStream_t);                                       \
   template cudaError_t launch_drag<T>(const StepArgs&, bool, const DragItem*, int, double*,        \
                                       cudaStream_t);                                               \
   template cudaError_t launch_audit<T>(const StepArgs&, double*, unsigned int*, double*, cudaStream_t); \

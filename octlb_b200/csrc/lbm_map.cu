@@ -396,6 +396,11 @@ cudaError_t launch_map_cm(const StepArgs& a, const NearTables& nt, bool links, b
 }
 }  // namespace
 
+// CTAs of a BGK step's launch.
+int map_step_ctas(const StepArgs& a, const NearTables& nt, bool links) {
+  return (links ? (nt.n + 3) / 4 : 0) + a.nblk * (a.n * a.n * a.n / 256) + (a.n_open + 127) / 128;
+}
+
 // One step of a level; cm: its collide.
 template <typename T>
 cudaError_t launch_step_map(const StepArgs& a, const NearTables& nt, bool links, bool flags, int cm, cudaStream_t s) {

@@ -66,14 +66,28 @@ void host_macro(const double* f, float out[23]) {
 template <typename T>
 int do_advance_level(octlb_ctx* ctx, int l);
 
-// Launches the pending restrictions (two per launch).
+// Whether a coupler launch lets the step of level L after it start early: its
+// CTAs then read their row tables while the coupler's finish (cylinder
+// 256x64x64, 2,445 CTAs on the finest level: 161 -> 155 us per call).  Not
+// where that step is one to two waves of the 8-CTA-per-SM form: CTAs placed
+// around the coupler's leave the SMs unevenly filled (AMR cavity, 1,077 and
+// 1,716 CTAs: 269 -> 276 us FP32, 234 -> 244 us FP16).
+bool couple_triggers(const octlb_ctx* ctx, const Level& L) {
+  if (!L.use_map || L.nblk == 0) return false;
+  const int ctas = map_step_ctas(L.args, L.near, ctx->stream_mode == OCTLB_STREAM_LINKS), sms = L.args.sms;
+  return ctas <= 5 * sms || ctas > 16 * sms;
+}
+
+// Launches the pending restrictions (two per launch) before the step of level
+// next (null: before anything else).
 template <typename T>
-int flush_restricts(octlb_ctx* ctx) {
+int flush_restricts(octlb_ctx* ctx, const Level* next = nullptr) {
   auto& P = ctx->pending_restrict;
   const ProlongOp none_p{};
   const RestrictOp none_r{};
   for (size_t k = 0; k < P.size(); k += 2) {
-    CK(launch_couple<T>(none_p, P[k].op, k + 1 < P.size() ? P[k + 1].op : none_r, ctx->stream));
+    CK(launch_couple<T>(none_p, P[k].op, k + 1 < P.size() ? P[k + 1].op : none_r,
+                        next && k + 2 >= P.size() && couple_triggers(ctx, *next), ctx->stream));
     ++ctx->launch_count;
   }
   P.clear();
@@ -90,7 +104,7 @@ int launch_level_step(octlb_ctx* ctx, Level& L) {
     if (int rc = fd_after_step<T>(ctx, L)) return rc;
     return exchange_rows(ctx, L);  // (slab contexts own every level's block)
   }
-  { const int rc = flush_restricts<T>(ctx); if (rc) return rc; }  // the step reads what they write
+  { const int rc = flush_restricts<T>(ctx, &L); if (rc) return rc; }  // the step reads what they write
   // Body force on the stored post-collision state (the reference's apply()
   // hook after collide, time_loop.h:207-211).  The boundary fills and the
   // same-level exchange that follow there need no launch: the step reads
@@ -257,7 +271,7 @@ int do_advance_level(octlb_ctx* ctx, int l) {
       if (!pend.empty()) r0 = pend[0].op;
       if (pend.size() > 1) r1 = pend[1].op;
       pend.clear();
-      CK(launch_couple<T>(p, r0, r1, ctx->stream));
+      CK(launch_couple<T>(p, r0, r1, couple_triggers(ctx, F), ctx->stream));
       ++ctx->launch_count;
     }
     rc = do_advance_level<T>(ctx, l + 1);

@@ -26,7 +26,8 @@ namespace octlb_gpu {
 
 template <typename T> cudaError_t launch_step(const StepArgs&, bool, bool, bool, cudaStream_t);
 template <typename T>
-cudaError_t launch_couple(const ProlongOp&, const RestrictOp&, const RestrictOp&, cudaStream_t);
+cudaError_t launch_couple(const ProlongOp&, const RestrictOp&, const RestrictOp&, bool, cudaStream_t);
+int map_step_ctas(const StepArgs&, const NearTables&, bool links);
 template <typename T>
 cudaError_t launch_drag(const StepArgs&, bool, const DragItem*, int, double*, cudaStream_t);
 cudaError_t launch_drag_total(const double*, int, double*, double*, cudaStream_t);
