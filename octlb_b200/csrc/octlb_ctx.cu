@@ -1199,7 +1199,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     CK(upload(L.nbase, nbase));
     CK(upload(L.page_of, page_of));
     CK(upload(L.hmap, hmap));
-    CK(upload(L.blk_gid, std::vector<int>(L.blocks.begin(), L.blocks.begin() + L.nblk)));
     CK(upload(L.hpos, hpos));
     CK(upload(L.open_items, open_items));
     CK(upload(L.near_cells, near_cells));
@@ -1464,8 +1463,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
   CK(ctx->drag_partial.alloc(static_cast<size_t>(std::max(ctx->drag_parts, 1)) * 3 * sizeof(double)));
   CK(ctx->force.alloc(3 * sizeof(double)));
   CK(ctx->force_sum.alloc(3 * sizeof(double)));
-  CK(ctx->audit_out.alloc(6 * sizeof(double) * nlev));
-  CK(ctx->audit_done.alloc(sizeof(unsigned int)));
 
   // ---- initial state: g = C(f0) on kBulk cells
   for (int l = 0; l < nlev && !g_dry_run && init; ++l) {
@@ -2049,6 +2046,77 @@ bool contiguous(const Level& L) {
   return true;
 }
 
+// bytes between a host array and device memory, in order on the context's
+// stream.  Pinned arrays, and small ones, are one cudaMemcpyAsync.  A large
+// pageable array goes through pinned buffers (HostStage) by several host
+// threads, a chunk each: the driver's own path copies it (and, into fresh
+// memory, takes its page faults) on one thread, 6.5 GB/s (110 MB each way of a
+// 90^3 box's restart: 34 ms).  Returns with the host array read or written.
+cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool to_device) {
+  const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+  auto plain = [&] {
+    const cudaError_t e = to_device ? cudaMemcpyAsync(dev, host, bytes, kind, ctx->stream)
+                                    : cudaMemcpyAsync(host, dev, bytes, kind, ctx->stream);
+    return e;
+  };
+  constexpr size_t kChunk = HostStage::kBytes;
+  cudaPointerAttributes attr{};
+  const bool pageable = bytes >= 8 * kChunk && cudaPointerGetAttributes(&attr, host) == cudaSuccess &&
+                        attr.type == cudaMemoryTypeUnregistered;
+  const unsigned cores = std::thread::hardware_concurrency();
+  if (!pageable || cores < 4) return plain();
+  if (ctx->host_stage.prepare() != cudaSuccess) {
+    cudaGetLastError();
+    return plain();
+  }
+  const std::unique_lock<std::mutex> hold(HostStage::shared().use, std::try_to_lock);
+  if (!hold.owns_lock()) return plain();
+  int device = 0;
+  if (cudaError_t e = cudaGetDevice(&device)) return e;
+  HostStage& hs = ctx->host_stage;
+  const size_t chunks = (bytes + kChunk - 1) / kChunk;
+  std::atomic<size_t> next{0};
+  std::atomic<int> error{0};
+  auto work = [&](int w) {
+    cudaError_t e = cudaSetDevice(device);
+    bool used = false;
+    while (e == cudaSuccess && error.load() == 0) {
+      const size_t k = next.fetch_add(1);
+      if (k >= chunks) break;
+      const size_t off = k * kChunk, n = std::min(kChunk, bytes - off);
+      char* h = static_cast<char*>(host) + off;
+      char* d = static_cast<char*>(dev) + off;
+      if (to_device) {
+        if (used) e = cudaEventSynchronize(hs.done[w]);  // the buffer's last copy has left it
+        if (e == cudaSuccess) {
+          std::memcpy(hs.buf(w), h, n);
+          e = cudaMemcpyAsync(d, hs.buf(w), n, kind, ctx->stream);
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(hs.done[w], ctx->stream);
+        used = true;
+      } else {
+        e = cudaMemcpyAsync(hs.buf(w), d, n, kind, ctx->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(hs.done[w], ctx->stream);
+        if (e == cudaSuccess) e = cudaEventSynchronize(hs.done[w]);
+        if (e == cudaSuccess) std::memcpy(h, hs.buf(w), n);
+      }
+    }
+    if (used && e == cudaSuccess) e = cudaEventSynchronize(hs.done[w]);
+    if (e != cudaSuccess) error.store(static_cast<int>(e));
+  };
+  std::vector<std::thread> threads;
+  const int helpers = std::min<int>(HostStage::kBufs, static_cast<int>(cores)) - 1;
+  try {
+    threads.reserve(helpers);
+    for (int w = 1; w <= helpers; ++w) threads.emplace_back(work, w);
+  } catch (const std::exception&) {
+    // no more threads: those that started, and this one, take all chunks
+  }
+  work(0);
+  for (std::thread& t : threads) t.join();
+  return static_cast<cudaError_t>(error.load());
+}
+
 // Whether set / get_populations and get_fields move all levels as one array in
 // the caller's block order, the kernels placing each level's blocks: one
 // context that owns every block, levels that are not runs of it, and staging
@@ -2059,7 +2127,11 @@ bool whole_array(octlb_ctx* ctx, size_t doubles_a, size_t doubles_b) {
   bool runs = true;
   for (const auto& L : ctx->levels) runs = runs && (L.nblk == 0 || contiguous(L));
   if (runs) return false;
-  if (ctx->stage_a.reserve(doubles_a * sizeof(double)) == cudaSuccess &&
+  bool ok = true;
+  for (auto& L : ctx->levels)  // the levels' block ids, made on first use
+    if (L.nblk > 0 && !L.blk_gid.p)
+      ok = ok && upload(L.blk_gid, std::vector<int>(L.blocks.begin(), L.blocks.begin() + L.nblk)) == cudaSuccess;
+  if (ok && ctx->stage_a.reserve(doubles_a * sizeof(double)) == cudaSuccess &&
       ctx->stage_b.reserve(doubles_b * sizeof(double)) == cudaSuccess)
     return true;
   cudaGetLastError();  // out of memory: level by level
@@ -2083,9 +2155,8 @@ int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
       if (!pops)
         if (int rc = fd_fix_fields(ctx, L, L.blk_gid.as<int>(), da, db)) return rc;
     }
-    CK(cudaMemcpyAsync(pops ? pops : rho, da, sizeof(double) * (pops ? all * kQ : all), cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    if (!pops) CK(cudaMemcpyAsync(u, db, sizeof(double) * all * 3, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(host_copy(ctx, pops ? pops : rho, da, sizeof(double) * (pops ? all * kQ : all), false));
+    if (!pops) CK(host_copy(ctx, u, db, sizeof(double) * all * 3, false));
     CK(cudaStreamSynchronize(ctx->stream));
     return OCTLB_OK;
   }
@@ -2115,8 +2186,8 @@ int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
       o0 = h0.data();
       if (mode == 1) { h1.resize(static_cast<size_t>(cells * 3)); o1 = h1.data(); }
     }
-    CK(cudaMemcpyAsync(o0, d.p, bytes0, cudaMemcpyDeviceToHost, ctx->stream));
-    if (mode == 1) CK(cudaMemcpyAsync(o1, du.p, bytes1, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(host_copy(ctx, o0, d.p, bytes0, false));
+    if (mode == 1) CK(host_copy(ctx, o1, du.p, bytes1, false));
     CK(cudaStreamSynchronize(ctx->stream));
     if (!direct) {
       for (int lb = 0; lb < L.nblk; ++lb) {
@@ -2139,7 +2210,7 @@ int scatter_impl(octlb_ctx* ctx, const double* in) {
   const size_t all = static_cast<size_t>(ctx->n_blocks * n3) * kQ;
   if (whole_array(ctx, all, 0)) {
     double* d = ctx->stage_a.as<double>();
-    CK(cudaMemcpyAsync(d, in, sizeof(double) * all, cudaMemcpyHostToDevice, ctx->stream));
+    CK(host_copy(ctx, const_cast<double*>(in), d, sizeof(double) * all, true));
     for (auto& L : ctx->levels) {
       if (L.nblk == 0) continue;
       StepArgs a = L.args;
@@ -2156,8 +2227,7 @@ int scatter_impl(octlb_ctx* ctx, const double* in) {
     const size_t bytes = static_cast<size_t>(cells * kQ) * sizeof(double);
     CK(d.reserve(bytes));
     if (contiguous(L)) {
-      CK(cudaMemcpyAsync(d.p, in + static_cast<long long>(L.blocks[0]) * n3 * kQ, bytes,
-                         cudaMemcpyHostToDevice, ctx->stream));
+      CK(host_copy(ctx, const_cast<double*>(in) + static_cast<long long>(L.blocks[0]) * n3 * kQ, d.p, bytes, true));
     } else {
       for (int lb = 0; lb < L.nblk; ++lb)
         CK(cudaMemcpyAsync(d.as<double>() + lb * n3 * kQ, in + static_cast<long long>(L.blocks[lb]) * n3 * kQ,
@@ -2184,8 +2254,8 @@ int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
   if (whole_array(ctx, all, all * 3)) {
     double* dr = ctx->stage_a.as<double>();
     double* du = ctx->stage_b.as<double>();
-    CK(cudaMemcpyAsync(dr, rho, sizeof(double) * all, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(du, u, sizeof(double) * 3 * all, cudaMemcpyHostToDevice, ctx->stream));
+    CK(host_copy(ctx, const_cast<double*>(rho), dr, sizeof(double) * all, true));
+    CK(host_copy(ctx, const_cast<double*>(u), du, sizeof(double) * 3 * all, true));
     for (auto& L : ctx->levels) {
       if (L.nblk == 0) continue;
       StepArgs a = L.args;
@@ -2204,8 +2274,8 @@ int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
     double* du = dr + cells;
     if (contiguous(L)) {
       const long long b0 = static_cast<long long>(L.blocks[0]) * n3;
-      CK(cudaMemcpyAsync(dr, rho + b0, sizeof(double) * cells, cudaMemcpyHostToDevice, ctx->stream));
-      CK(cudaMemcpyAsync(du, u + 3 * b0, sizeof(double) * 3 * cells, cudaMemcpyHostToDevice, ctx->stream));
+      CK(host_copy(ctx, const_cast<double*>(rho) + b0, dr, sizeof(double) * cells, true));
+      CK(host_copy(ctx, const_cast<double*>(u) + 3 * b0, du, sizeof(double) * 3 * cells, true));
     } else {
       for (int lb = 0; lb < L.nblk; ++lb) {
         const long long b0 = static_cast<long long>(L.blocks[lb]) * n3;
@@ -2235,6 +2305,10 @@ int audit_impl(octlb_ctx* ctx, double out[4]) {
   for (auto& L : ctx->levels)
     if (L.nblk > 0) parts = std::max<size_t>(parts, audit_partials(L.args));
   CK(ctx->audit_partial.reserve(parts * 5 * sizeof(double)));
+  if (!ctx->audit_done.p) {
+    CK(ctx->audit_out.alloc(6 * sizeof(double) * nl));
+    CK(ctx->audit_done.alloc(sizeof(unsigned int)));
+  }
   for (size_t l = 0; l < nl; ++l) {
     Level& L = ctx->levels[l];
     if (L.nblk == 0) continue;

@@ -5,6 +5,7 @@
 #pragma once
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -16,6 +17,8 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <unordered_set>
 #include <vector>
 
@@ -23,6 +26,61 @@
 #include "../../include/octlb_gpu.h"
 
 namespace octlb_gpu {
+
+// Pinned buffers between pageable host arrays and the device, one per copying
+// thread (octlb_ctx.cu, host_copy).  The memory (8 MB; pinning it takes about
+// 1 ms per MB) is one region per process, made on first use, shared by the
+// contexts that have used it -- one copy at a time, a second one meanwhile
+// takes the driver's path -- and freed with the last of them.  The events are
+// the context's own.
+struct HostStage {
+  static constexpr int kBufs = 8;
+  static constexpr size_t kBytes = 1u << 20;
+  struct Shared {
+    std::mutex use, count;  // the copy that holds the buffers; users and mem
+    int users = 0;
+    char* mem = nullptr;
+  };
+  static Shared& shared() {
+    static Shared* s = new Shared;  // outlives every context, also at exit
+    return *s;
+  }
+  cudaEvent_t done[kBufs] = {};
+  bool user = false;
+  char* buf(int i) const { return shared().mem + i * kBytes; }
+  cudaError_t prepare() {
+    if (user) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < kBufs && e == cudaSuccess; ++i)
+      if (!done[i]) e = cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    Shared& s = shared();
+    const std::lock_guard<std::mutex> lock(s.count);
+    if (!s.mem) {
+      void* p = nullptr;
+      e = cudaHostAlloc(&p, kBufs * kBytes, cudaHostAllocPortable);
+      if (e != cudaSuccess) return e;
+      s.mem = static_cast<char*>(p);
+    }
+    ++s.users;
+    user = true;
+    return cudaSuccess;
+  }
+  HostStage() = default;
+  HostStage(const HostStage&) = delete;
+  HostStage& operator=(const HostStage&) = delete;
+  ~HostStage() {
+    for (cudaEvent_t e : done)
+      if (e) cudaEventDestroy(e);
+    if (!user) return;
+    Shared& s = shared();
+    const std::lock_guard<std::mutex> lock(s.count);
+    if (--s.users == 0) {
+      cudaFreeHost(s.mem);
+      s.mem = nullptr;
+    }
+  }
+};
 
 template <typename T> cudaError_t launch_step(const StepArgs&, bool, bool, bool, cudaStream_t);
 template <typename T>
@@ -322,6 +380,7 @@ struct octlb_ctx {
   // FP64 host-layout staging of set/get_populations and get_fields (grown on
   // demand, kept until destroy: no allocation per call)
   DevBuf stage_a, stage_b;
+  HostStage host_stage;
   int drag_parts = 0;
   long long force_steps = 0;
   std::vector<int> counters_collide, counters_stream;
