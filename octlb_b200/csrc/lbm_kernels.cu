@@ -944,6 +944,9 @@ __global__ void __launch_bounds__(kThreads) k_collide_cr(const StepArgs a, float
 __global__ void __launch_bounds__(kThreads)
 k_cr_update(double* avg, const double* part, int nparts, long long count, const double* bpart, int nbparts,
             long long bcount, float* shift) {
+  // one CTA: the step's may start beside it and read their tables (they wait
+  // for the average)
+  pdl_trigger();
   pdl_wait();
   double v[2] = {0.0, 0.0};
   for (int p = threadIdx.x; p < nparts; p += kThreads) v[0] += part[p];
