@@ -1463,6 +1463,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
   CK(ctx->drag_partial.alloc(static_cast<size_t>(std::max(ctx->drag_parts, 1)) * 3 * sizeof(double)));
   CK(ctx->force.alloc(3 * sizeof(double)));
   CK(ctx->force_sum.alloc(3 * sizeof(double)));
+  CK(ctx->audit_out.alloc((6 * nlev + 1) * sizeof(double)));  // per level 5 sums and the error word; the CTA count
 
   // ---- initial state: g = C(f0) on kBulk cells
   for (int l = 0; l < nlev && !g_dry_run && init; ++l) {
@@ -2305,17 +2306,14 @@ int audit_impl(octlb_ctx* ctx, double out[4]) {
   for (auto& L : ctx->levels)
     if (L.nblk > 0) parts = std::max<size_t>(parts, audit_partials(L.args));
   CK(ctx->audit_partial.reserve(parts * 5 * sizeof(double)));
-  if (!ctx->audit_done.p) {
-    CK(ctx->audit_out.alloc(6 * sizeof(double) * nl));
-    CK(ctx->audit_done.alloc(sizeof(unsigned int)));
-  }
   for (size_t l = 0; l < nl; ++l) {
     Level& L = ctx->levels[l];
     if (L.nblk == 0) continue;
     StepArgs a = L.args;
     a.src = L.buf[L.cur].p;
     a.aa_rev = L.aa && L.cur;
-    CK(launch_audit<T>(a, ctx->audit_partial.as<double>(), ctx->audit_done.as<unsigned int>(),
+    CK(launch_audit<T>(a, ctx->audit_partial.as<double>(),
+                       reinterpret_cast<unsigned int*>(ctx->audit_out.as<double>() + 6 * nl),
                        ctx->audit_out.as<double>() + 6 * l, ctx->stream));
   }
   std::vector<double> h(6 * nl);  // per level the 5 sums and the error word

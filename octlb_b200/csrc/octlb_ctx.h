@@ -376,7 +376,7 @@ struct octlb_ctx {
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   bool side_busy = false;
-  DevBuf drag_partial, force, force_sum, audit_out, audit_partial, audit_done, host_tmp, dev_err;
+  DevBuf drag_partial, force, force_sum, audit_out, audit_partial, host_tmp, dev_err;
   // FP64 host-layout staging of set/get_populations and get_fields (grown on
   // demand, kept until destroy: no allocation per call)
   DevBuf stage_a, stage_b;
