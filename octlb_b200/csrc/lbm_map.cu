@@ -231,16 +231,12 @@ __global__ void __launch_bounds__(THREADS, WARPS * 32 / THREADS) k_step_map(cons
       f[combo_dn(c)] = raw2<SM>(shift_down(dn, h[c], zhi, wall), inv);
     }
     if (info & kBlkMoving) {
-      // wall term k = -marker - 2; moving rows have consecutive ones (the table
-      // is read again: in L1, and no registers held)
+      // wall term k = -marker - 2 (the table is read again: in L1, and no
+      // registers held)
 #pragma unroll
       for (int i = 1; i < kQ; ++i) {
-        const int m = __ldg(rm - (cx(i) * kNp + cy(i)));
-        int m0 = (cx(i) || cy(i)) && m < -1 ? m - (static_cast<int>(z) - cz(i)) : 0, m1 = m0 - (m0 < -1);
-        if (cz(i) != 0) {
-          if (cz(i) > 0 && zlo) m0 = __ldg(rm + kRow - (cx(i) * kNp + cy(i)));
-          if (cz(i) < 0 && zhi) m1 = __ldg(rm + 2 * kRow - (cx(i) * kNp + cy(i)));
-        }
+        int m0, m1;
+        row_wall_marks(cx(i) || cy(i), rm - (cx(i) * kNp + cy(i)), kRow, cz(i), static_cast<int>(z), N, m0, m1);
         float u, v;
         upk(f[i], u, v);
         if (m0 < -1) u += a.wall_add[(-m0 - 2) * kQ + i] * wscale;

@@ -1304,6 +1304,29 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
             if (!wall && !run && !same) info[lb] &= static_cast<uint8_t>(~kBlkRows);
           }
       }
+      // Planning only: every position that a pair of cells pulls, as the step's
+      // row path forms it, against the slot map itself.
+      for (int lb = 0; g_dry_run && lb < L.nblk; ++lb) {
+        if (!(info[lb] & kBlkRows)) continue;
+        const int* m = slot_map.data() + static_cast<size_t>(lb) * np3;
+        for (int x = 0; x < n; ++x)
+          for (int y = 0; y < n; ++y)
+            for (int z = 0; z < n; z += 2)
+              for (int i = 1; i < kQ; ++i) {
+                const int at = (x + 1 - cx(i)) * np + y + 1 - cy(i);
+                const int* rs = row_map.data() + static_cast<size_t>(lb) * 3 * np * np + at;
+                int mark[2];
+                row_wall_marks(cx(i) || cy(i), rs, np * np, cz(i), z, n, mark[0], mark[1]);
+                for (int k = 0; k < 2; ++k) {
+                  const uint8_t f = flags[static_cast<size_t>(core_slot_of(n, lb, x, y, z + k))];
+                  if (links && ((f & kKindMask) == kSolid || (f & kFlagNear))) continue;
+                  const int Z = z + 1 + k - cz(i), want = m[at * np + Z];
+                  const int got = Z == 0 ? rs[np * np] : (Z > n ? rs[2 * np * np] : (rs[0] >= 0 ? rs[0] + Z - 1 : (rs[0] == -1 ? -1 : mark[k])));
+                  if (got != want || (want < -1 ? want : 0) != (mark[k] < -1 ? mark[k] : 0))
+                    return fail(ctx, OCTLB_EINVAL, "internal: row table disagrees with the slot map");
+                }
+              }
+      }
       CK(upload(L.blk_info, info));
       CK(upload(L.row_map, row_map));
       A.row_map = L.row_map.as<int>();
