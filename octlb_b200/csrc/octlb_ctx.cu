@@ -2088,7 +2088,9 @@ cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool 
   const bool pageable = bytes >= 8 * kChunk && cudaPointerGetAttributes(&attr, host) == cudaSuccess &&
                         attr.type == cudaMemoryTypeUnregistered;
   const unsigned cores = std::thread::hardware_concurrency();
-  if (!pageable || cores < 4) return plain();
+  // The per-thread default stream's handle names another stream in each thread:
+  // a helper's copies would run beside the kernels they have to wait for.
+  if (!pageable || cores < 4 || ctx->stream == cudaStreamPerThread) return plain();
   if (ctx->host_stage.prepare() != cudaSuccess) {
     cudaGetLastError();
     return plain();
