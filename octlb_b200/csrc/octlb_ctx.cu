@@ -2070,6 +2070,46 @@ bool contiguous(const Level& L) {
   return true;
 }
 
+// Whether the calling thread's current context is the current device's primary
+// one, the one a helper thread gets from cudaSetDevice (and the only one whose
+// pinned buffers every context of the process can share for good).
+bool primary_context() {
+  using GetCurrent = int (*)(void**);
+  using GetState = int (*)(int, unsigned*, int*);
+  using Retain = int (*)(void**, int);
+  using Release = int (*)(int);
+  struct Api {
+    GetCurrent current = nullptr;
+    GetState state = nullptr;
+    Retain retain = nullptr;
+    Release release = nullptr;
+    Api() {
+      auto get = [](const char* name, unsigned version) {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion(name, &f, version, cudaEnableDefault, &q) != cudaSuccess) {
+          cudaGetLastError();
+          return static_cast<void*>(nullptr);
+        }
+        return q == cudaDriverEntryPointSuccess ? f : nullptr;
+      };
+      current = reinterpret_cast<GetCurrent>(get("cuCtxGetCurrent", 12000));
+      state = reinterpret_cast<GetState>(get("cuDevicePrimaryCtxGetState", 12000));
+      retain = reinterpret_cast<Retain>(get("cuDevicePrimaryCtxRetain", 12000));
+      release = reinterpret_cast<Release>(get("cuDevicePrimaryCtxRelease", 12000));
+    }
+  };
+  static const Api api;
+  if (!api.current || !api.state || !api.retain || !api.release) return false;
+  int dev = 0, active = 0;
+  unsigned flags = 0;
+  void *cur = nullptr, *primary = nullptr;
+  if (cudaGetDevice(&dev) != cudaSuccess || api.current(&cur) != 0 || !cur) return false;
+  if (api.state(dev, &flags, &active) != 0 || !active || api.retain(&primary, dev) != 0) return false;
+  api.release(dev);
+  return cur == primary;
+}
+
 // bytes between a host array and device memory, in order on the context's
 // stream.  Pinned arrays, and small ones, are one cudaMemcpyAsync.  A large
 // pageable array goes through pinned buffers (HostStage) by several host
@@ -2091,6 +2131,7 @@ cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool 
   // The per-thread default stream's handle names another stream in each thread:
   // a helper's copies would run beside the kernels they have to wait for.
   if (!pageable || cores < 4 || ctx->stream == cudaStreamPerThread) return plain();
+  if (!primary_context()) return plain();
   if (ctx->host_stage.prepare() != cudaSuccess) {
     cudaGetLastError();
     return plain();
