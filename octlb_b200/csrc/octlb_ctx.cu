@@ -691,14 +691,19 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
   std::vector<int> hmap(static_cast<size_t>(np3), -1), hpos;
   for (int pass = 0; pass < 2; ++pass)
     for (int X = 0; X < np; ++X)
-      for (int Y = 0; Y < np; ++Y)
-        for (int Z = 0; Z < np; ++Z) {
-          const bool core = X >= 1 && Y >= 1 && Z >= 1 && X <= n && Y <= n && Z <= n;
-          if (core || (Z >= 1 && Z <= n) != (pass == 0)) continue;
+      for (int Y = 0; Y < np; ++Y) {
+        const bool core = X >= 1 && Y >= 1 && X <= n && Y <= n;  // a row of core cells but for its two ends
+        if (pass == 0 && core) continue;
+        for (int Z = pass == 0 ? 1 : 0; Z < np; Z += pass == 0 ? 1 : n + 1) {
+          if (pass == 0 && Z > n) break;
           hmap[(X * np + Y) * np + Z] = static_cast<int>(hpos.size());
           hpos.push_back((X * np + Y) * np + Z);
         }
+      }
   const int H = static_cast<int>(hpos.size());
+  std::vector<int> by_pos;  // the halo indices in order of padded position
+  for (int P = 0; P < np3 && !ctx->periodic; ++P)
+    if (hmap[P] >= 0) by_pos.push_back(hmap[P]);
   auto dir27 = [&](int X, int Y, int Z) {
     const int ox = X == 0 ? -1 : (X == n + 1 ? 1 : 0), oy = Y == 0 ? -1 : (Y == n + 1 ? 1 : 0),
               oz = Z == 0 ? -1 : (Z == n + 1 ? 1 : 0);
@@ -792,13 +797,16 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     // exchange), in list order; a later write of the same halo population
     // wins.  Keyed by (block, padded position, population).
     struct BB { int lb, hlin, pop; long long src; int src_pop; float add, dadd; };
-    std::map<std::tuple<int, int, int>, size_t> bbidx;
+    std::vector<std::vector<int>> fill_at(static_cast<size_t>(L.nblk));  // per block with fills: [H][kQ] index in bbl, or -1
     std::vector<BB> bbl;
+    auto filled = [&](int lb, int hlin, int pop) {
+      return !fill_at[lb].empty() && hmap[hlin] >= 0 && fill_at[lb][static_cast<size_t>(hmap[hlin]) * kQ + pop] >= 0;
+    };
     auto put_bb = [&](int lb, int hlin, int pop, long long src, int src_pop, float add, float dadd) {
-      const auto key = std::make_tuple(lb, hlin, pop);
-      auto it = bbidx.find(key);
-      if (it == bbidx.end()) { bbidx.emplace(key, bbl.size()); bbl.push_back({lb, hlin, pop, src, src_pop, add, dadd}); }
-      else bbl[it->second] = {lb, hlin, pop, src, src_pop, add, dadd};
+      if (fill_at[lb].empty()) fill_at[lb].assign(static_cast<size_t>(H) * kQ, -1);
+      int& at = fill_at[lb][static_cast<size_t>(hmap[hlin]) * kQ + pop];
+      if (at < 0) { at = static_cast<int>(bbl.size()); bbl.push_back({lb, hlin, pop, src, src_pop, add, dadd}); }
+      else bbl[at] = {lb, hlin, pop, src, src_pop, add, dadd};
     };
     for (int k = 0; k < t->n_tree_boundary; ++k) {
       const int gb = t->tree_boundary[2 * k], dir = t->tree_boundary[2 * k + 1];
@@ -855,7 +863,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
       auto covered = [&](int lb, int X, int Y, int Z, int pop) {
         const int d = dir27(X, Y, Z);
         if (nbr27[static_cast<size_t>(lb) * 27 + d] >= 0) return true;
-        return bbidx.count(std::make_tuple(lb, (X * np + Y) * np + Z, pop)) > 0;
+        return filled(lb, (X * np + Y) * np + Z, pop);
       };
       for (int lb = 0; lb < L.nblk; ++lb) {
         bool open = false;
@@ -895,15 +903,18 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
       auto covered = [&](int lb, int hlin, int pop) {
         const int X = hlin / (np * np), Y = (hlin / np) % np, Z = hlin % np;
         if (nbr27[static_cast<size_t>(lb) * 27 + dir27(X, Y, Z)] >= 0) return true;
-        return bbidx.count(std::make_tuple(lb, hlin, pop)) > 0;
+        return filled(lb, hlin, pop);
       };
       for (int lb = 0; lb < L.nblk; ++lb) {
         if (!is_open[lb]) continue;
-        std::set<std::pair<int, int>> need;
+        std::vector<char> need(static_cast<size_t>(H) * kQ, 0);
         std::vector<std::pair<int, int>> work;
         auto add = [&](int hlin, int pop) {
-          if (hmap[hlin] < 0 || covered(lb, hlin, pop)) return;
-          if (need.insert({hlin, pop}).second) work.push_back({hlin, pop});
+          if (hmap[hlin] < 0) return;
+          char& in = need[static_cast<size_t>(hmap[hlin]) * kQ + pop];
+          if (in || covered(lb, hlin, pop)) return;
+          in = 1;
+          work.push_back({hlin, pop});
         };
         for (int x = 1; x <= n; ++x)
           for (int y = 1; y <= n; ++y)
@@ -924,12 +935,14 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
           src = ((src % np3) + np3) % np3;
           add(src, pop);
         }
-        for (const auto& hp : need) {
-          halo_items.push_back(page_of[lb]);
-          halo_items.push_back(lb);
-          halo_items.push_back(hmap[hp.first]);
-          halo_items.push_back(hp.second);
-        }
+        for (int h : by_pos)
+          for (int pop = 0; pop < kQ; ++pop)
+            if (need[static_cast<size_t>(h) * kQ + pop]) {
+              halo_items.push_back(page_of[lb]);
+              halo_items.push_back(lb);
+              halo_items.push_back(h);
+              halo_items.push_back(pop);
+            }
       }
     }
     L.n_open = static_cast<int>(halo_items.size() / 4);
@@ -977,8 +990,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     };
     // The halo items resolved: page slot written, slot its torus pull reads
     // (block_lattice.h:70-89), population, 1 where that source is a fill.
-    std::vector<int> open_items;
-    open_items.reserve(halo_items.size());
+    std::vector<int> open_items(halo_items.size());
     for (size_t k = 0; k < halo_items.size(); k += 4) {
       const int lb = halo_items[k + 1], hidx = halo_items[k + 2], pop = halo_items[k + 3];
       int sp = hpos[hidx] - (cx(pop) * np * np + cy(pop) * np + cz(pop));
@@ -988,7 +1000,10 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
       if (from < 0 || from >= L.nslots || to >= L.nslots || L.nslots > INT_MAX)
         return fail(ctx, OCTLB_EINVAL, "internal: halo item without a source");
       const bool fill = from >= core_end && fill_of_h[static_cast<size_t>(from - core_end) * kQ + pop] >= 0;
-      open_items.insert(open_items.end(), {static_cast<int>(to), static_cast<int>(from), pop, fill ? 1 : 0});
+      open_items[k] = static_cast<int>(to);
+      open_items[k + 1] = static_cast<int>(from);
+      open_items[k + 2] = pop;
+      open_items[k + 3] = fill ? 1 : 0;
     }
     std::vector<int> slot_map;
     std::vector<float> wall_add, wall_dadd;  // per moving-wall position: the 19 wall terms, their velocity derivative
