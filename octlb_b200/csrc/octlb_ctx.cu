@@ -2139,9 +2139,9 @@ cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool 
     return e;
   };
   constexpr size_t kChunk = HostStage::kBytes;
+  if (bytes < 8 * kChunk) return plain();  // (the queries below take a tenth of a small call)
   cudaPointerAttributes attr{};
-  const bool pageable = bytes >= 8 * kChunk && cudaPointerGetAttributes(&attr, host) == cudaSuccess &&
-                        attr.type == cudaMemoryTypeUnregistered;
+  const bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
   const unsigned cores = std::thread::hardware_concurrency();
   // The per-thread default stream's handle names another stream in each thread:
   // a helper's copies would run beside the kernels they have to wait for.
