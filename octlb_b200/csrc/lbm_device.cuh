@@ -92,6 +92,15 @@ __device__ __forceinline__ float pull_value(const StepArgs& a, const T* src, int
   return Store<T>::ld(src + i * a.qs + s, a.inv_scale);
 }
 
+// Cell t of the level in the host arrays of a run, -1 where its block is not in
+// the run: block-local order kept.
+__device__ __forceinline__ long long host_cell(const BlockRun& run, const FastDiv& div_n3, uint32_t t) {
+  if (!run.gid) return t;
+  const uint32_t b = div_n3.div(t);
+  const int k = run.gid[b] - run.first;
+  return k >= 0 && k < run.count ? static_cast<long long>(k) * div_n3.d + (t - b * div_n3.d) : -1;
+}
+
 // Halo item k of an open block (block_lattice.h:70-89), resolved on the host:
 // the page slot it writes, the slot its torus pull reads (own core, the
 // neighbour core the exchange copies, or the own halo page), its population,

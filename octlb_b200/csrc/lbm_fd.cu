@@ -446,7 +446,7 @@ k_fd_rows_from_state(const T* state, long long qs, float inv_s, const FdCell* ce
 // over the fields the gather wrote; the bounce-back cells' fields are the
 // gathered ones (their streamed state).
 __global__ void __launch_bounds__(kFdThreads)
-k_fd_fields(const FdCell* cells, int n, const float* fnew, const int* gid, FastDiv div_n3, double* rho, double* u) {
+k_fd_fields(const FdCell* cells, int n, const float* fnew, const BlockRun run, FastDiv div_n3, double* rho, double* u) {
   const int row = blockIdx.x * kFdThreads + threadIdx.x;
   if (row >= n || cells[row].role == 0) return;
   double dr = 0, jx = 0, jy = 0, jz = 0;
@@ -457,8 +457,8 @@ k_fd_fields(const FdCell* cells, int n, const float* fnew, const int* gid, FastD
   }
   const double r = 1.0 + dr;
   // the cell in the host arrays, as k_gather placed it
-  const uint32_t t = static_cast<uint32_t>(cells[row].slot), b = div_n3.div(t);
-  const long long s = gid ? static_cast<long long>(gid[b]) * div_n3.d + (t - b * div_n3.d) : t;
+  const long long s = host_cell(run, div_n3, static_cast<uint32_t>(cells[row].slot));
+  if (s < 0) return;
   rho[s] = r;
   u[3 * s] = jx / r;
   u[3 * s + 1] = jy / r;
@@ -507,10 +507,10 @@ cudaError_t launch_fd_rows_from_state(const void* state, long long qs, float inv
   return cudaGetLastError();
 }
 
-cudaError_t launch_fd_fields(const FdCell* cells, int n, const float* fnew, const int* gid, FastDiv div_n3, double* rho,
+cudaError_t launch_fd_fields(const FdCell* cells, int n, const float* fnew, const BlockRun& run, FastDiv div_n3, double* rho,
                              double* u, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  k_fd_fields<<<fd_grid(n), kFdThreads, 0, s>>>(cells, n, fnew, gid, div_n3, rho, u);
+  k_fd_fields<<<fd_grid(n), kFdThreads, 0, s>>>(cells, n, fnew, run, div_n3, rho, u);
   return cudaGetLastError();
 }
 

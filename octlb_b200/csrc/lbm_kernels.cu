@@ -761,25 +761,18 @@ k_audit(const StepArgs a, double* partial, unsigned int* done, double* out) {
   }
 }
 
-// Cell t of the level in the host arrays: block-local order kept, its block at
-// gid[block] (null: the level's blocks are the arrays' blocks in order).  With
-// gid a forest's levels go to and come from one array in the caller's block
-// order, and one copy moves it: reordering on the host cost 40 ms of a 512x128x
-// 128 cylinder's get_fields (94 MB, pageable buffers), the one copy takes 2.
-__device__ __forceinline__ long long host_cell(const StepArgs& a, const int* gid, uint32_t t) {
-  if (!gid) return t;
-  const uint32_t b = a.div_n3.div(t);
-  return static_cast<long long>(gid[b]) * (a.n * a.n * a.n) + (t - b * a.n * a.n * a.n);
-}
-
-// Core cells <-> dense FP64 host order [block][ix][iy][iz][19].
+// Core cells <-> dense FP64 host order [block][ix][iy][iz][19].  A forest's
+// levels go to and come from one array in the caller's block order (BlockRun):
+// reordering on the host cost 40 ms of a 512x128x128 cylinder's get_fields (94
+// MB, pageable buffers), the copies without it 2.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_gather(const StepArgs a, double* out, double* out_u, const int* gid, int mode /*0 pops, 1 fields*/) {
+k_gather(const StepArgs a, double* out, double* out_u, const BlockRun run, int mode /*0 pops, 1 fields*/) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   if (t >= a.ncore) return;
   const long long slot = t;  // compact core slot
-  const long long hc = host_cell(a, gid, t);
+  const long long hc = host_cell(run, a.div_n3, t);
+  if (hc < 0) return;
   const T* src = static_cast<const T*>(a.src);
   if (mode == 0) {
 #pragma unroll
@@ -805,15 +798,19 @@ k_gather(const StepArgs a, double* out, double* out_u, const int* gid, int mode 
 // Reference state f (pre-collision, FP64) -> stored g = C(f) for kBulk cells.
 // Under ConstRhoBGK the collide is taken at *cr_avg, and each CTA's sum of
 // rho - 1 over its kBulk cells goes to cr_part[blockIdx.x] (the statistics of
-// that collide; the near-wall partials after them, near_parts, are zeroed).
+// that collide; the near-wall partials after them, near_parts, are zeroed).  A
+// level's blocks outside the run are left as they are, and with the statistics
+// a CTA's cells are then one block's (scatter_runs).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_scatter(const StepArgs a, const double* in, const int* gid, int near_parts) {
+k_scatter(const StepArgs a, const double* in, const BlockRun run, int near_parts) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   double v[1] = {0.0};
+  const long long hc = t < a.ncore ? host_cell(run, a.div_n3, t) : -1;
+  if (run.gid && hc < 0) return;
   if (t < a.ncore) {
     const long long slot = t;  // compact core slot
-    const double* hp = in + host_cell(a, gid, t) * kQ;
+    const double* hp = in + hc * kQ;
     float f[kQ];
 #pragma unroll
     for (int i = 0; i < kQ; ++i) f[i] = static_cast<float>(hp[i]);
@@ -843,12 +840,13 @@ k_scatter(const StepArgs a, const double* in, const int* gid, int near_parts) {
 // equilibrium formed on the host in that order.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-k_scatter_eq(const StepArgs a, const double* in_rho, const double* in_u, const int* gid, int near_parts) {
+k_scatter_eq(const StepArgs a, const double* in_rho, const double* in_u, const BlockRun run, int near_parts) {
   const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
   double v[1] = {0.0};
+  const long long hc = t < a.ncore ? host_cell(run, a.div_n3, t) : -1;
+  if (run.gid && hc < 0) return;
   if (t < a.ncore) {
     const long long slot = t;
-    const long long hc = host_cell(a, gid, t);
     const double rho = in_rho[hc];
     const double* up = in_u + 3 * hc;
     const double ux = up[0], uy = up[1], uz = up[2];
@@ -1115,21 +1113,23 @@ cudaError_t launch_audit(const StepArgs& a, double* partial, unsigned int* done,
   return cudaGetLastError();
 }
 uint32_t audit_partials(const StepArgs& a) { return grid_for(a.ncore); }
+// Whether no CTA of a launch over cells holds cells of two blocks.
+bool block_of_whole_ctas(int n) { return n * n * n % kThreads == 0; }
 
 template <typename T>
-cudaError_t launch_gather(const StepArgs& a, double* out, double* out_u, const int* gid, int mode, cudaStream_t s) {
-  k_gather<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, out, out_u, gid, mode);
+cudaError_t launch_gather(const StepArgs& a, double* out, double* out_u, const BlockRun& run, int mode, cudaStream_t s) {
+  k_gather<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, out, out_u, run, mode);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_scatter(const StepArgs& a, const double* in, const int* gid, int near_parts, cudaStream_t s) {
-  k_scatter<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, in, gid, near_parts);
+cudaError_t launch_scatter(const StepArgs& a, const double* in, const BlockRun& run, int near_parts, cudaStream_t s) {
+  k_scatter<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, in, run, near_parts);
   return cudaGetLastError();
 }
 template <typename T>
-cudaError_t launch_scatter_eq(const StepArgs& a, const double* rho, const double* u, const int* gid, int near_parts,
+cudaError_t launch_scatter_eq(const StepArgs& a, const double* rho, const double* u, const BlockRun& run, int near_parts,
                               cudaStream_t s) {
-  k_scatter_eq<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, rho, u, gid, near_parts);
+  k_scatter_eq<T><<<grid_for(a.ncore), kThreads, 0, s>>>(a, rho, u, run, near_parts);
   return cudaGetLastError();
 }
 
@@ -1195,9 +1195,9 @@ cudaError_t launch_cr_update(double* avg, const double* part, int nparts, long l
   template cudaError_t launch_drag<T>(const StepArgs&, bool, const DragItem*, int, double*,        \
                                       cudaStream_t);                                               \
   template cudaError_t launch_audit<T>(const StepArgs&, double*, unsigned int*, double*, cudaStream_t); \
-  template cudaError_t launch_gather<T>(const StepArgs&, double*, double*, const int*, int, cudaStream_t);  \
-  template cudaError_t launch_scatter<T>(const StepArgs&, const double*, const int*, int, cudaStream_t); \
-  template cudaError_t launch_scatter_eq<T>(const StepArgs&, const double*, const double*, const int*, int, cudaStream_t); \
+  template cudaError_t launch_gather<T>(const StepArgs&, double*, double*, const BlockRun&, int, cudaStream_t);  \
+  template cudaError_t launch_scatter<T>(const StepArgs&, const double*, const BlockRun&, int, cudaStream_t); \
+  template cudaError_t launch_scatter_eq<T>(const StepArgs&, const double*, const double*, const BlockRun&, int, cudaStream_t); \
   template cudaError_t launch_step_cr<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
   template cudaError_t launch_step_nc<T>(const StepArgs&, const NearTables&, bool, bool, cudaStream_t); \
   template cudaError_t launch_collide_cr<T>(const StepArgs&, float*, cudaStream_t);                \

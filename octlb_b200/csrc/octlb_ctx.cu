@@ -1515,7 +1515,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     CK(upload(d, dense));
     StepArgs a = L.args;
     a.dst = L.buf[L.cur].p;
-    CK(launch_scatter<T>(a, d.as<double>(), nullptr, 0, ctx->stream));
+    CK(launch_scatter<T>(a, d.as<double>(), BlockRun{}, 0, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
   }
   long long lups = 0;
@@ -2199,46 +2199,61 @@ cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool 
   return static_cast<cudaError_t>(error.load());
 }
 
-// Whether set / get_populations and get_fields move all levels as one array in
-// the caller's block order, the kernels placing each level's blocks: one
-// context that owns every block, levels that are not runs of it, and staging
-// for all of it (a single level, or levels in block order, needs no reordering
-// and stages level by level; so does a forest whose whole staging does not fit).
-bool whole_array(octlb_ctx* ctx, size_t doubles_a, size_t doubles_b) {
-  if (!ctx->owner.empty()) return false;
+// The blocks per run in which set / get_populations, set_equilibrium and
+// get_fields move a forest's levels together in the caller's block order, the
+// kernels placing each level's blocks (BlockRun): as many as the largest level
+// has, so a run's staging is what that level alone would take.  0: level by
+// level -- rank contexts, and levels that are runs of the caller's order already.
+int run_blocks(const octlb_ctx* ctx) {
+  if (!ctx->owner.empty()) return 0;
   bool runs = true;
-  for (const auto& L : ctx->levels) runs = runs && (L.nblk == 0 || contiguous(L));
-  if (runs) return false;
-  bool ok = true;
-  for (auto& L : ctx->levels)  // the levels' block ids, made on first use
-    if (L.nblk > 0 && !L.blk_gid.p)
-      ok = ok && upload(L.blk_gid, std::vector<int>(L.blocks.begin(), L.blocks.begin() + L.nblk)) == cudaSuccess;
-  if (ok && ctx->stage_a.reserve(doubles_a * sizeof(double)) == cudaSuccess &&
-      ctx->stage_b.reserve(doubles_b * sizeof(double)) == cudaSuccess)
-    return true;
-  cudaGetLastError();  // out of memory: level by level
-  ctx->stage_a.alloc(0);
-  ctx->stage_b.alloc(0);
-  return false;
+  int most = 0;
+  for (const auto& L : ctx->levels) {
+    runs = runs && (L.nblk == 0 || contiguous(L));
+    most = std::max(most, L.nblk);
+  }
+  return runs ? 0 : most;
+}
+
+// ... for the state's writers: under ConstRhoBGK they also sum the statistics
+// CTA by CTA, which takes a block of whole CTAs.
+int scatter_runs(const octlb_ctx* ctx) {
+  return ctx->const_rho && !block_of_whole_ctas(ctx->n) ? 0 : run_blocks(ctx);
+}
+
+// Level L's part of the run of `most` blocks from `first` (its block ids go to
+// the device on first use).
+cudaError_t level_run(octlb_ctx* ctx, Level& L, int first, int most, BlockRun& run) {
+  if (!L.blk_gid.p)
+    if (cudaError_t e = upload(L.blk_gid, std::vector<int>(L.blocks.begin(), L.blocks.begin() + L.nblk))) return e;
+  run = BlockRun{L.blk_gid.as<int>(), first, std::min(most, ctx->n_blocks - first)};
+  return cudaSuccess;
 }
 
 template <typename T>
 int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
   const long long n3 = static_cast<long long>(ctx->n) * ctx->n * ctx->n;
-  const size_t all = static_cast<size_t>(ctx->n_blocks * n3);
-  if (whole_array(ctx, pops ? all * kQ : all, pops ? 0 : all * 3)) {
+  if (const int most = run_blocks(ctx)) {
+    CK(ctx->stage_a.reserve(static_cast<size_t>(most * n3 * (pops ? kQ : 1)) * sizeof(double)));
+    if (!pops) CK(ctx->stage_b.reserve(static_cast<size_t>(most * n3 * 3) * sizeof(double)));
     double* da = ctx->stage_a.as<double>();
     double* db = ctx->stage_b.as<double>();
-    for (auto& L : ctx->levels) {
-      if (L.nblk == 0) continue;
-      StepArgs a = L.args;
-      a.src = L.buf[L.cur].p;
-      CK(launch_gather<T>(a, da, db, L.blk_gid.as<int>(), pops ? 0 : 1, ctx->stream));
-      if (!pops)
-        if (int rc = fd_fix_fields(ctx, L, L.blk_gid.as<int>(), da, db)) return rc;
+    for (int first = 0; first < ctx->n_blocks; first += most) {
+      for (auto& L : ctx->levels) {
+        if (L.nblk == 0) continue;
+        BlockRun run;
+        CK(level_run(ctx, L, first, most, run));
+        StepArgs a = L.args;
+        a.src = L.buf[L.cur].p;
+        CK(launch_gather<T>(a, da, db, run, pops ? 0 : 1, ctx->stream));
+        if (!pops)
+          if (int rc = fd_fix_fields(ctx, L, run, da, db)) return rc;
+      }
+      const long long c0 = first * n3;
+      const size_t cells = static_cast<size_t>(std::min(most, ctx->n_blocks - first) * n3);
+      CK(host_copy(ctx, pops ? pops + c0 * kQ : rho + c0, da, sizeof(double) * (pops ? cells * kQ : cells), false));
+      if (!pops) CK(host_copy(ctx, u + c0 * 3, db, sizeof(double) * cells * 3, false));
     }
-    CK(host_copy(ctx, pops ? pops : rho, da, sizeof(double) * (pops ? all * kQ : all), false));
-    if (!pops) CK(host_copy(ctx, u, db, sizeof(double) * all * 3, false));
     CK(cudaStreamSynchronize(ctx->stream));
     return OCTLB_OK;
   }
@@ -2255,9 +2270,9 @@ int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
     StepArgs a = L.args;
     a.src = L.buf[L.cur].p;
     a.aa_rev = L.aa && L.cur;
-    CK(launch_gather<T>(a, d.as<double>(), du.as<double>(), nullptr, mode, ctx->stream));
+    CK(launch_gather<T>(a, d.as<double>(), du.as<double>(), BlockRun{}, mode, ctx->stream));
     if (mode == 1)  // the FD pass's Dirichlet cells: the fields of their rewritten rows
-      if (int rc = fd_fix_fields(ctx, L, nullptr, d.as<double>(), du.as<double>())) return rc;
+      if (int rc = fd_fix_fields(ctx, L, BlockRun{}, d.as<double>(), du.as<double>())) return rc;
     const bool direct = contiguous(L);
     const long long off = static_cast<long long>(L.blocks[0]) * n3;
     std::vector<double> h0, h1;
@@ -2289,15 +2304,20 @@ int gather_impl(octlb_ctx* ctx, double* pops, double* rho, double* u) {
 template <typename T>
 int scatter_impl(octlb_ctx* ctx, const double* in) {
   const long long n3 = static_cast<long long>(ctx->n) * ctx->n * ctx->n;
-  const size_t all = static_cast<size_t>(ctx->n_blocks * n3) * kQ;
-  if (whole_array(ctx, all, 0)) {
+  if (const int most = scatter_runs(ctx)) {
+    CK(ctx->stage_a.reserve(static_cast<size_t>(most * n3 * kQ) * sizeof(double)));
     double* d = ctx->stage_a.as<double>();
-    CK(host_copy(ctx, const_cast<double*>(in), d, sizeof(double) * all, true));
-    for (auto& L : ctx->levels) {
-      if (L.nblk == 0) continue;
-      StepArgs a = L.args;
-      a.dst = L.buf[L.cur].p;
-      CK(launch_scatter<T>(a, d, L.blk_gid.as<int>(), a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    for (int first = 0; first < ctx->n_blocks; first += most) {
+      const size_t cells = static_cast<size_t>(std::min(most, ctx->n_blocks - first) * n3);
+      CK(host_copy(ctx, const_cast<double*>(in) + first * n3 * kQ, d, sizeof(double) * cells * kQ, true));
+      for (auto& L : ctx->levels) {
+        if (L.nblk == 0) continue;
+        BlockRun run;
+        CK(level_run(ctx, L, first, most, run));
+        StepArgs a = L.args;
+        a.dst = L.buf[L.cur].p;
+        CK(launch_scatter<T>(a, d, run, a.cr_part ? ctx->cr_near : 0, ctx->stream));
+      }
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return OCTLB_OK;
@@ -2317,7 +2337,7 @@ int scatter_impl(octlb_ctx* ctx, const double* in) {
     }
     StepArgs a = L.args;
     a.dst = L.buf[L.cur].p;
-    CK(launch_scatter<T>(a, d.as<double>(), nullptr, a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    CK(launch_scatter<T>(a, d.as<double>(), BlockRun{}, a.cr_part ? ctx->cr_near : 0, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (L.aa) L.cur = 0;  // the natural layout again
   }
@@ -2332,17 +2352,24 @@ int scatter_impl(octlb_ctx* ctx, const double* in) {
 template <typename T>
 int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
   const long long n3 = static_cast<long long>(ctx->n) * ctx->n * ctx->n;
-  const size_t all = static_cast<size_t>(ctx->n_blocks * n3);
-  if (whole_array(ctx, all, all * 3)) {
+  if (const int most = scatter_runs(ctx)) {
+    CK(ctx->stage_a.reserve(static_cast<size_t>(most * n3) * sizeof(double)));
+    CK(ctx->stage_b.reserve(static_cast<size_t>(most * n3 * 3) * sizeof(double)));
     double* dr = ctx->stage_a.as<double>();
     double* du = ctx->stage_b.as<double>();
-    CK(host_copy(ctx, const_cast<double*>(rho), dr, sizeof(double) * all, true));
-    CK(host_copy(ctx, const_cast<double*>(u), du, sizeof(double) * 3 * all, true));
-    for (auto& L : ctx->levels) {
-      if (L.nblk == 0) continue;
-      StepArgs a = L.args;
-      a.dst = L.buf[L.cur].p;
-      CK(launch_scatter_eq<T>(a, dr, du, L.blk_gid.as<int>(), a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    for (int first = 0; first < ctx->n_blocks; first += most) {
+      const long long c0 = first * n3;
+      const size_t cells = static_cast<size_t>(std::min(most, ctx->n_blocks - first) * n3);
+      CK(host_copy(ctx, const_cast<double*>(rho) + c0, dr, sizeof(double) * cells, true));
+      CK(host_copy(ctx, const_cast<double*>(u) + c0 * 3, du, sizeof(double) * 3 * cells, true));
+      for (auto& L : ctx->levels) {
+        if (L.nblk == 0) continue;
+        BlockRun run;
+        CK(level_run(ctx, L, first, most, run));
+        StepArgs a = L.args;
+        a.dst = L.buf[L.cur].p;
+        CK(launch_scatter_eq<T>(a, dr, du, run, a.cr_part ? ctx->cr_near : 0, ctx->stream));
+      }
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return OCTLB_OK;
@@ -2368,7 +2395,7 @@ int scatter_eq_impl(octlb_ctx* ctx, const double* rho, const double* u) {
     }
     StepArgs a = L.args;
     a.dst = L.buf[L.cur].p;
-    CK(launch_scatter_eq<T>(a, dr, du, nullptr, a.cr_part ? ctx->cr_near : 0, ctx->stream));
+    CK(launch_scatter_eq<T>(a, dr, du, BlockRun{}, a.cr_part ? ctx->cr_near : 0, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (L.aa) L.cur = 0;  // the natural layout again
   }

@@ -90,10 +90,10 @@ template <typename T>
 cudaError_t launch_drag(const StepArgs&, bool, const DragItem*, int, double*, cudaStream_t);
 cudaError_t launch_drag_total(const double*, int, double*, double*, cudaStream_t);
 template <typename T> cudaError_t launch_audit(const StepArgs&, double*, unsigned int*, double*, cudaStream_t);
-template <typename T> cudaError_t launch_gather(const StepArgs&, double*, double*, const int*, int, cudaStream_t);
-template <typename T> cudaError_t launch_scatter(const StepArgs&, const double*, const int*, int, cudaStream_t);
+template <typename T> cudaError_t launch_gather(const StepArgs&, double*, double*, const BlockRun&, int, cudaStream_t);
+template <typename T> cudaError_t launch_scatter(const StepArgs&, const double*, const BlockRun&, int, cudaStream_t);
 template <typename T>
-cudaError_t launch_scatter_eq(const StepArgs&, const double*, const double*, const int*, int, cudaStream_t);
+cudaError_t launch_scatter_eq(const StepArgs&, const double*, const double*, const BlockRun&, int, cudaStream_t);
 template <typename T>
 cudaError_t launch_step_cr(const StepArgs&, const NearTables&, bool, bool, cudaStream_t);
 template <typename T> cudaError_t launch_cr_seed(const StepArgs&, int, cudaStream_t);
@@ -134,6 +134,7 @@ cudaError_t launch_adj_restrict(const RestrictItem*, int, const float*, float*, 
 bool bulk_step_eligible(int n, int elem_bytes);
 uint32_t drag_partials(int n);
 uint32_t audit_partials(const StepArgs& a);
+bool block_of_whole_ctas(int n);
 
 // Host-only planning (octlb_gpu_plan): every allocation, upload and launch is
 // skipped while the tables are flattened and checked.
@@ -488,7 +489,7 @@ template <typename T> int fd_after_step(octlb_ctx* ctx, Level& L);
 template <typename T> int fd_before_step(octlb_ctx* ctx, Level& L);
 int fd_end_of_step(octlb_ctx* ctx);
 bool fd_updates_average(const octlb_ctx* ctx, const Level& L);
-int fd_fix_fields(octlb_ctx* ctx, Level& L, const int* gid, double* rho, double* u);
+int fd_fix_fields(octlb_ctx* ctx, Level& L, const BlockRun& run, double* rho, double* u);
 void clear_graphs(octlb_ctx* ctx);
 void comm_detach(octlb_ctx* ctx);
 

@@ -27,7 +27,7 @@ unsigned fd_collide_parts(int n);
 cudaError_t launch_fd_tick(double*, cudaStream_t);
 template <typename T>
 cudaError_t launch_fd_rows_from_state(const void*, long long, float, const FdCell*, int, float*, cudaStream_t);
-cudaError_t launch_fd_fields(const FdCell*, int, const float*, const int*, FastDiv, double*, double*, cudaStream_t);
+cudaError_t launch_fd_fields(const FdCell*, int, const float*, const BlockRun&, FastDiv, double*, double*, cudaStream_t);
 template <typename T>
 cudaError_t launch_fd_store(void*, long long, float, const FdCell*, int, const float*, double*, double, cudaStream_t);
 }  // namespace octlb_gpu
@@ -222,9 +222,9 @@ template int fd_after_step<__half>(octlb_ctx*, Level&);
 
 // get_fields: the Dirichlet cells' rho and u from their rows (level L's
 // staging arrays, indexed by local core slot).
-int fd_fix_fields(octlb_ctx* ctx, Level& L, const int* gid, double* rho, double* u) {
+int fd_fix_fields(octlb_ctx* ctx, Level& L, const BlockRun& run, double* rho, double* u) {
   if (!ctx->fd_on || L.nblk == 0 || L.fd_rows == 0) return OCTLB_OK;
-  CK(launch_fd_fields(L.fd_cells.as<FdCell>(), L.fd_rows, L.fd_new.as<float>(), gid, L.args.div_n3, rho, u,
+  CK(launch_fd_fields(L.fd_cells.as<FdCell>(), L.fd_rows, L.fd_new.as<float>(), run, L.args.div_n3, rho, u,
                       ctx->stream));
   return OCTLB_OK;
 }

@@ -130,6 +130,14 @@ __host__ __device__ __forceinline__ void row_wall_marks(bool off_axis, const int
 
 constexpr long long kOwnPage = -(1LL << 62);
 
+// Host arrays in the caller's block order that hold blocks first .. first +
+// count - 1 of it: block b of the level is global block gid[b].  gid null: the
+// arrays hold the level's own blocks, in its order.
+struct BlockRun {
+  const int* gid = nullptr;
+  int first = 0, count = 0;
+};
+
 // Device error codes written to StepArgs::err.
 // kErrBulkDrainTimeout: a CTA that gave up could not see its own copies in
 // flight land either, so shared memory may still be written after it exited.
