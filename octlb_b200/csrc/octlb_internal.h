@@ -116,14 +116,14 @@ __host__ __device__ __forceinline__ int table_entry(const int* p) {
 // cells (z, z + 1) pulls in a direction with c_z = cz.  rs[0], rs[plane] and
 // rs[2 plane] are the row table's entries of the source row at Z = 1, 0 and
 // n + 1; off_axis: it is not the pair's own row.  A marker below -1 is a moving
-// wall, anything else a position without a wall term.  Each marker is formed
-// on its own: one of the two may lie beyond the row.
+// wall, anything else a position without a wall term.  (m1 follows from whether
+// the row moves, not from m0's value: m0 may lie beyond the row.)
 __host__ __device__ __forceinline__ void row_wall_marks(bool off_axis, const int* rs, int plane, int cz, int z, int n, int& m0,
                                                         int& m1) {
   const int row = table_entry(rs);
   const bool moving = off_axis && row < -1;
   m0 = moving ? row - (z - cz) : 0;
-  m1 = moving ? row - (z + 1 - cz) : 0;
+  m1 = moving ? m0 - 1 : 0;
   if (cz > 0 && z == 0) m0 = table_entry(rs + plane);
   if (cz < 0 && z == n - 2) m1 = table_entry(rs + 2 * plane);
 }
