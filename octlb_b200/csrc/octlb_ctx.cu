@@ -2139,9 +2139,15 @@ cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool 
     return e;
   };
   constexpr size_t kChunk = HostStage::kBytes;
-  if (bytes < 8 * kChunk) return plain();  // (the queries below take a tenth of a small call)
+  // Small arrays to the device go straight: the queries below are 5 us of host
+  // time per array (set_equilibrium of a 32^3 box: 102 us with them, 90 without).
+  // Small ones from it follow a kernel, and that time passes beside it; a copy
+  // queued before the kernel's end costs more than one queued after it (advance,
+  // audit and get_fields of a 32^3 box: 96.5 us with the queries, 101 without).
+  if (to_device && bytes < 8 * kChunk) return plain();
   cudaPointerAttributes attr{};
-  const bool pageable = cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
+  const bool pageable = bytes >= 8 * kChunk && cudaPointerGetAttributes(&attr, host) == cudaSuccess &&
+                        attr.type == cudaMemoryTypeUnregistered;
   const unsigned cores = std::thread::hardware_concurrency();
   // The per-thread default stream's handle names another stream in each thread:
   // a helper's copies would run beside the kernels they have to wait for.
