@@ -107,11 +107,14 @@ __device__ __forceinline__ long long host_cell(const BlockRun& run, const FastDi
 // and whether that source is a tree-boundary fill.  (Resolved here, an item was
 // a chain of five dependent reads: halo index, position, base or page, value.)
 __device__ __forceinline__ bool rotate_slots(const StepArgs& a, uint32_t k, long long& dst, long long& src, int& i) {
-  const int4 it = __ldg(reinterpret_cast<const int4*>(a.open_items) + k);
-  dst = it.x;
-  src = it.y;
-  i = it.z;
-  return it.w != 0;
+  static_assert(sizeof(OpenItem) == sizeof(int4), "one 16-byte load");
+  const int4 v = __ldg(reinterpret_cast<const int4*>(a.open_items) + k);
+  OpenItem it;
+  memcpy(&it, &v, sizeof(it));
+  dst = it.to();
+  src = it.from();
+  i = it.pop;
+  return it.fill != 0;
 }
 
 // Lane-parallel forms (lane i < 19 holds population i): lattice vectors and

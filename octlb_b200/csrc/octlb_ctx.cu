@@ -990,20 +990,17 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     };
     // The halo items resolved: page slot written, slot its torus pull reads
     // (block_lattice.h:70-89), population, 1 where that source is a fill.
-    std::vector<int> open_items(halo_items.size());
+    std::vector<OpenItem> open_items(halo_items.size() / 4);
     for (size_t k = 0; k < halo_items.size(); k += 4) {
       const int lb = halo_items[k + 1], hidx = halo_items[k + 2], pop = halo_items[k + 3];
       int sp = hpos[hidx] - (cx(pop) * np * np + cy(pop) * np + cz(pop));
       sp = ((sp % np3) + np3) % np3;
       const long long to = core_end + static_cast<long long>(halo_items[k]) * H + hidx;
       const long long from = resolve_slot(lb, sp / (np * np), (sp / np) % np, sp % np);
-      if (from < 0 || from >= L.nslots || to >= L.nslots || L.nslots > INT_MAX)
+      if (from < 0 || from >= L.nslots || to >= L.nslots || L.nslots > kOpenItemSlots)
         return fail(ctx, OCTLB_EINVAL, "internal: halo item without a source");
       const bool fill = from >= core_end && fill_of_h[static_cast<size_t>(from - core_end) * kQ + pop] >= 0;
-      open_items[k] = static_cast<int>(to);
-      open_items[k + 1] = static_cast<int>(from);
-      open_items[k + 2] = pop;
-      open_items[k + 3] = fill ? 1 : 0;
+      open_items[k / 4] = open_item(to, from, pop, fill);
     }
     std::vector<int> slot_map;
     std::vector<float> wall_add, wall_dadd;  // per moving-wall position: the 19 wall terms, their velocity derivative
@@ -1163,8 +1160,8 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
           return fail(ctx, OCTLB_EINVAL, "internal: boundary fill out of range");
       for (int v : lidx) if (v < -1 || v >= L.n_links) return fail(ctx, OCTLB_EINVAL, "internal: link index");
       for (int v : sidx) if (v < -1 || v >= L.n_save) return fail(ctx, OCTLB_EINVAL, "internal: save index");
-      for (size_t k = 0; k < open_items.size(); k += 4)
-        if (!in(open_items[k], ns) || open_items[k] < core_end || !in(open_items[k + 1], ns) || !in(open_items[k + 2], kQ))
+      for (const OpenItem& it : open_items)
+        if (!in(it.to(), ns) || it.to() < core_end || !in(it.from(), ns) || !in(it.pop, kQ))
           return fail(ctx, OCTLB_EINVAL, "internal: halo item");
       for (int lb = 0; lb < L.nblk; ++lb)
         for (int d = 0; d < 27; ++d) {
@@ -1254,7 +1251,7 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     A.page_of = L.page_of.as<int>();
     A.hmap = L.hmap.as<int>();
     A.hpos = L.hpos.as<int>();
-    A.open_items = L.open_items.as<int>();
+    A.open_items = L.open_items.as<OpenItem>();
     A.n_open = L.n_open;
     A.n_halo = L.n_halo;
     A.nblk = L.nblk; A.n = n; A.np = np;
@@ -2891,6 +2888,16 @@ int octlb_gpu_plan_part(const octlb_tables* t, const octlb_params* p, int rank, 
 // Host-only check of the multiply-high divider the kernels use for index
 // decomposition (no device work).
 unsigned octlb_gpu_debug_fastdiv(unsigned d, unsigned n) { return FastDiv(d).div(n); }
+
+// Host-only check of the halo items' slot fields: out = {written, read,
+// population, fill} as a kernel reads them back.
+void octlb_gpu_debug_open_item(long long to, long long from, int pop, int fill, long long out[4]) {
+  const OpenItem it = open_item(to, from, pop, fill != 0);
+  out[0] = it.to();
+  out[1] = it.from();
+  out[2] = it.pop;
+  out[3] = it.fill;
+}
 
 int octlb_gpu_step_stats(const octlb_ctx* ctx, long long* launches, long long* lups) {
   if (!ctx) return OCTLB_EINVAL;

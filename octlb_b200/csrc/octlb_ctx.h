@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
-#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>

@@ -33,7 +33,7 @@ struct StepArgs {
   const int* page_of;       // [nblk] halo page or -1
   const int* hmap;          // [(n+2)^3] padded position -> halo index (-1 in the core)
   const int* hpos;          // [n_halo] halo index -> padded linear position
-  const int* open_items;    // [n_open][4] torus-streamed halo items: slot written, slot read, population, 1: a fill is read
+  const struct OpenItem* open_items; // [n_open] torus-streamed halo items
   const int* slot_map;      // [nblk][(n+2)^3] slot of every padded position (k_step_map levels)
   const int* row_map;       // [nblk][3][(n+2)^2] slot map at Z = 1, 0 and n + 1 (kBlkRows blocks)
   const int* fill_of;       // [n_pages * n_halo][19] boundary fill writing (page slot, population), or -1
@@ -129,6 +129,22 @@ __host__ __device__ __forceinline__ void row_wall_marks(bool off_axis, const int
 }
 
 constexpr long long kOwnPage = -(1LL << 62);
+
+// A torus-streamed halo item of an open block (StepArgs::open_items): the slot
+// written, the slot read, the population, and whether a fill is read there.
+// Slots have 48 bits (a level in FP16 may have more than 2^31).
+struct alignas(16) OpenItem {
+  uint32_t dst, src;
+  uint16_t dst_hi, src_hi;
+  uint16_t pop, fill;
+  __host__ __device__ long long to() const { return static_cast<long long>(dst_hi) << 32 | dst; }
+  __host__ __device__ long long from() const { return static_cast<long long>(src_hi) << 32 | src; }
+};
+constexpr long long kOpenItemSlots = 1LL << 48;
+inline OpenItem open_item(long long to, long long from, int pop, bool fill) {
+  return OpenItem{static_cast<uint32_t>(to), static_cast<uint32_t>(from), static_cast<uint16_t>(to >> 32),
+                  static_cast<uint16_t>(from >> 32), static_cast<uint16_t>(pop), static_cast<uint16_t>(fill)};
+}
 
 // Host arrays in the caller's block order that hold blocks first .. first +
 // count - 1 of it: block b of the level is global block gid[b].  gid null: the
