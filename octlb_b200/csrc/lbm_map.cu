@@ -382,11 +382,16 @@ cudaError_t launch_map(const StepArgs& a, const NearTables& nt, bool links, bool
   const uint32_t parts = N * N * N / (2 * kT);
   const uint32_t near_ctas = links ? (static_cast<uint32_t>(nt.n) + kT / 32 - 1) / (kT / 32) : 0;
   const dim3 g(near_ctas + static_cast<uint32_t>(a.nblk) * parts + (static_cast<uint32_t>(a.n_open) + kT - 1) / kT);
-  // 32 warps per SM (64 registers, the loads in two batches, some spills) win
-  // where the CTAs fill more than one wave of the 20-warp form (2.1M cells FP32:
-  // 63.8 us against 74.6); that form issues every load at once and wins where
-  // they do not (32^3 cells: 4.1 us per step against 5.1).
-  const bool wide = g.x * (kT / 32) <= 20u * static_cast<uint32_t>(a.sms);
+  // 32 warps per SM (64 registers, the loads in two batches, 40 - 150 bytes of
+  // spill) win where the CTAs fill more than one wave of the 20-warp form (2.1M
+  // cells FP32: 63.8 us against 74.6); that form issues every load at once and
+  // wins where they do not (32^3 cells: 4.1 us per step against 5.1).  It holds
+  // five 128-thread CTAs per SM, and two of the statistics' 256-thread ones (16
+  // warps): ConstRhoBGK on 324 - 360 blocks of 8^3, 7.7 us per step with 32 warps
+  // against 9.4 - 9.8 FP32, 7.2 - 7.3 against 7.8 - 8.0 FP16; on 288 - 294 blocks
+  // 6.7 - 6.9 and 5.8 - 6.0 us with the 20-warp form.
+  constexpr uint32_t kResident = 20 * 32 / kT;
+  const bool wide = g.x <= kResident * static_cast<uint32_t>(a.sms);
   if constexpr (SM != kConvert)
     if (wide) return launch_map_w<T, N, SM, CM, 20>(a, nt, links, flags, g, s);
   return launch_map_w<T, N, SM, CM, 32>(a, nt, links, flags, g, s);
