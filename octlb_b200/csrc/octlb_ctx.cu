@@ -2158,7 +2158,7 @@ cudaError_t host_copy(octlb_ctx* ctx, void* host, void* dev, size_t bytes, bool 
   // The per-thread default stream's handle names another stream in each thread:
   // a helper's copies would run beside the kernels they have to wait for.
   if (!pageable || cores < 4 || ctx->stream == cudaStreamPerThread) return plain();
-  if (!primary_context()) return plain();
+  if (!primary_context() || !ctx->host_stage.repaid(bytes, to_device)) return plain();
   if (ctx->host_stage.prepare() != cudaSuccess) {
     cudaGetLastError();
     return plain();
