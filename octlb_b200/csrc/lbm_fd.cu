@@ -471,10 +471,6 @@ inline unsigned fd_grid(int n) { return static_cast<unsigned>((n + kFdThreads - 
 
 unsigned fd_collide_parts(int n) { return fd_grid(n); }
 
-namespace {
-
-}  // namespace
-
 template <typename T>
 cudaError_t launch_fd_reconstruct(const void* state, long long qs, float inv_s, const FdCell* cells, const int* list,
                                   int role, int n, float* fnew, const double* time, double time_shift, float omega,

@@ -1,5 +1,5 @@
-// A pair of cells in packed FP32 (f32x2) registers: loads, stores and the
-// collide of the kernels that hold two cells per thread.
+// A pair of cells in packed FP32 (f32x2) registers: the arithmetic and the
+// collide of the slot-map step, which holds two cells per thread.
 #ifndef OCTLB_LBM_PAIR_CUH_
 #define OCTLB_LBM_PAIR_CUH_
 
@@ -126,23 +126,6 @@ __device__ __forceinline__ void collide2(u64 (&f)[kQ], float omega, float s, flo
     both(16, cu_pos<16>(ux, uy, uz)); both(17, cu_pos<17>(ux, uy, uz)); both(18, cu_pos<18>(ux, uy, uz));
   }
 }
-
-// Stored values (FP16: storage units) as floats, and back.
-__device__ __forceinline__ float ld_raw(const float* p) { return *p; }
-__device__ __forceinline__ float ld_raw(const __half* p) { return __half2float(*p); }
-__device__ __forceinline__ u64 ld_pair(const float* p) { return *reinterpret_cast<const u64*>(p); }
-__device__ __forceinline__ u64 ld_pair(const __half* p) {
-  const float2 w = __half22float2(*reinterpret_cast<const __half2*>(p));
-  return pk(w.x, w.y);
-}
-__device__ __forceinline__ void st_pair(float* p, u64 v) { *reinterpret_cast<u64*>(p) = v; }
-__device__ __forceinline__ void st_pair(__half* p, u64 v) {
-  float a, b;
-  upk(v, a, b);
-  *reinterpret_cast<__half2*>(p) = __floats2half2_rn(a, b);
-}
-__device__ __forceinline__ void st_raw(float* p, float v) { *p = v; }
-__device__ __forceinline__ void st_raw(__half* p, float v) { *p = __float2half_rn(v); }
 
 }  // namespace
 }  // namespace octlb_gpu

@@ -1,5 +1,5 @@
 // Parts of the level step shared by the step kernels (lbm_kernels.cu,
-// lbm_map.cu): solid-cell copies, halo items of open blocks, near-wall cells.
+// lbm_map.cuh): solid-cell copies, halo items of open blocks, near-wall cells.
 #ifndef OCTLB_LBM_STEP_CUH_
 #define OCTLB_LBM_STEP_CUH_
 

@@ -1220,7 +1220,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     CK(upload(L.nbase, nbase));
     CK(upload(L.page_of, page_of));
     CK(upload(L.hmap, hmap));
-    CK(upload(L.hpos, hpos));
     CK(upload(L.open_items, open_items));
     CK(upload(L.near_cells, near_cells));
     CK(upload(L.near_mask, nmask));
@@ -1259,7 +1258,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     A.nbase = L.nbase.as<long long>();
     A.page_of = L.page_of.as<int>();
     A.hmap = L.hmap.as<int>();
-    A.hpos = L.hpos.as<int>();
     A.open_items = L.open_items.as<OpenItem>();
     A.n_open = L.n_open;
     A.n_halo = L.n_halo;
@@ -1271,9 +1269,6 @@ int create_impl(octlb_ctx* ctx, const octlb_tables* t, const octlb_params* p, co
     A.div_n = FastDiv(n);
     A.div_n2 = FastDiv(n * n);
     A.div_n3 = FastDiv(static_cast<uint32_t>(n3));
-    A.div_halo = FastDiv(L.n_halo > 0 ? L.n_halo : 1);
-    A.div_np = FastDiv(np);
-    A.div_np2 = FastDiv(np * np);
     A.omega = static_cast<float>(ctx->omega_l[l]);
     A.scale = L.scale;
     A.inv_scale = L.inv_scale;

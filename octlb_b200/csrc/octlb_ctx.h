@@ -226,7 +226,7 @@ struct Level {
   int cur = 0;
   DevBuf blk_gid;                   // [nblk] global block id
   DevBuf flags, link_idx, link_rec, save_idx, save_buf;
-  DevBuf nbase, page_of, hmap, hpos, open_items, near_cells, slot_map, row_map;
+  DevBuf nbase, page_of, hmap, open_items, near_cells, slot_map, row_map;
   DevBuf near_mask, near_slot, near_q, near_add;
   NearTables near{};
   int n_near = 0;

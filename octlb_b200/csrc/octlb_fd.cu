@@ -149,6 +149,10 @@ struct Builder {
 
 namespace octlb_host {
 
+// The boundary clock of the current step: steps of one graph behind the first
+// count from the clock at its start (single-level meshes; others tick per step).
+double fd_shift(const octlb_ctx* ctx) { return ctx->fd_single ? ctx->batch_pos : 0.0; }
+
 // The pass after a step of level S: the reference's apply_post_stream()
 // after each level's stream -- an empty level's too -- runs it on every
 // tree-boundary block of every level (domain_boundary_handler.cpp:81-93,
@@ -156,10 +160,6 @@ namespace octlb_host {
 // planes, edges, corners into the rows, then the rows into the state,
 // uncollided, as the reference rewrites the cells in place -- a later pass
 // on a level that has not stepped since reads them as its "pre" values.
-// The boundary clock of the current step: steps of one graph behind the first
-// count from the clock at its start (single-level meshes; others tick per step).
-double fd_shift(const octlb_ctx* ctx) { return ctx->fd_single ? ctx->batch_pos : 0.0; }
-
 template <typename T>
 int fd_after_step(octlb_ctx* ctx, Level& S) {
   (void)S;

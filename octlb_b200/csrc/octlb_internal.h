@@ -32,7 +32,6 @@ struct StepArgs {
   const long long* nbase;   // [nblk][27] slot base of the halo direction (or kOwnPage)
   const int* page_of;       // [nblk] halo page or -1
   const int* hmap;          // [(n+2)^3] padded position -> halo index (-1 in the core)
-  const int* hpos;          // [n_halo] halo index -> padded linear position
   const struct OpenItem* open_items; // [n_open] torus-streamed halo items
   const int* slot_map;      // [nblk][(n+2)^3] slot of every padded position (k_step_map levels)
   const int* row_map;       // [nblk][3][(n+2)^2] slot map at Z = 1, 0 and n + 1 (kBlkRows blocks)
@@ -47,7 +46,7 @@ struct StepArgs {
   long long halo_base;      // first halo-page slot (= nblk * n^3)
   uint32_t ncore;           // nblk * n^3 core work items
   uint32_t nitems;          // ncore + n_open
-  FastDiv div_n, div_n2, div_n3, div_halo, div_np, div_np2;
+  FastDiv div_n, div_n2, div_n3;
   float omega, scale, inv_scale;
   int off[kQ];              // core slot offset of c_i: cx*n*n + cy*n + cz
   int off_pad[kQ];          // padded linear offset of c_i: cx*np*np + cy*np + cz
