@@ -292,9 +292,12 @@ __device__ __forceinline__ void st4h(__half* p, float a, float b, float c, float
 // Launches of the time-step chain: with the programmatic stream-serialisation
 // attribute when enabled, so each kernel is launched as its predecessor's
 // CTAs exit and runs its constant-table prologue before pdl_wait (every such
-// kernel calls pdl_wait before its first dependent access).  No kernel
-// triggers its dependents early: measured on the forest cases, an early
-// trigger gained nothing over the implicit trigger at CTA exit.
+// kernel calls pdl_wait before its first dependent access).  The small kernels
+// of the chain also trigger their dependents early -- the FD pass's
+// (lbm_fd.cu), the average update, the coupler's where couple_triggers says so,
+// and the coupler's and drag's adjoints, each with its figures; a dependent still
+// waits for the whole grid.  The step kernels do not: their successors' CTAs
+// would take the places of their own (64^3 AMR cavity 269 -> 283 us per call).
 template <typename... P, typename... A>
 cudaError_t launch_chain(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg{};

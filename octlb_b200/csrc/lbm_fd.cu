@@ -30,7 +30,7 @@
 // records (constant tables, two dependent reads) before it waits for its
 // predecessor, so what remains of a launch on the critical path is one read of
 // the state, the arithmetic and one write.  cavity3d's 31^3 step: 43.8 us in
-// plain stream order with a launch for the average and a store per step, 31.9 us now.
+// plain stream order with a launch for the average and a store per step, 32.2 us now.
 #include "lbm_device.cuh"
 
 namespace octlb_gpu {
