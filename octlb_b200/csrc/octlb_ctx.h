@@ -49,12 +49,11 @@ struct HostStage {
     static Shared* s = new Shared;  // outlives every context, also at exit
     return *s;
   }
-  static constexpr size_t kRepaid = 48u << 20;  // bytes from the device that win the pinning back
+  static constexpr size_t kRepaid = 32u << 20;  // bytes from the device that win the pinning back
   cudaEvent_t done[kBufs] = {};
   bool user = false;
   size_t moved = 0;  // by the driver's path so far, in bytes from the device's worth
   bool repaid(size_t bytes, bool to_device) {
-    if (user) return true;
     {
       const std::lock_guard<std::mutex> lock(shared().count);
       if (shared().mem) return true;

@@ -13,7 +13,7 @@ def ob():
 
 
 @pytest.mark.parametrize("beside", [False, True])
-@pytest.mark.parametrize("n", [40, 64])  # populations of 9.7 and 39.8 MB: the fifth and second copy back change the path
+@pytest.mark.parametrize("n", [40, 64])  # populations of 9.7 and 39.8 MB: the third and first copy back change the path
 def test_same_bytes_on_both_paths(ob, n, beside):
     rng = np.random.default_rng(n)
     mesh = ob.Mesh(n, [0], [0, 0, 0, 1, 1, 1], periodic=1)
