@@ -71,14 +71,15 @@ int do_advance_level(octlb_ctx* ctx, int l);
 // around the coupler's leave the SMs unevenly filled, which costs most where the
 // step is between one wave of the 20-warp form (5 CTAs per SM) and two of the
 // 32-warp one (16).  us per call with no early start, with it before every step,
-// and with it outside that range (CTAs per SM of the finest level):
-//   64^3 cavity, band 8 (6.9), FP32 270.1 / 275.3 / 270.1, FP16 228.6 / 239.2 / 228.8
-//   band 16 (13.8)             422.7 / 417.3 / 419.2,      293.8 / 296.5 / 296.6
-//   band 24 (20.8)             567.0 / 560.3 / 561.0,      384.6 / 383.0 / 384.1
-//   32^3 cavity, band 8 (1.7)   66.1 /  68.0 /  68.0,       66.0 /  64.6 /  64.5
-//   band 16 (3.5)               75.1 /  74.1 /  74.2,       72.1 /  71.6 /  72.0
-//   cylinder 256x64x64 (16.5)  160.7 / 156.2 / 156.1,      129.8 / 128.0 / 127.8
-//   refined less far (13)      129.3 / 127.6 / 128.8,      117.9 / 116.7 / 117.5
+// and with it outside that range (CTAs per SM of each level's step):
+//   64^3 cavity, band 8 (7, 12), FP32 270.1 / 275.3 / 270.1, FP16 228.6 / 239.2 / 228.8
+//   band 16 (6, 19)              422.7 / 417.3 / 419.2,      293.8 / 296.5 / 296.6
+//   band 24 (5.5, 25)            567.0 / 560.3 / 561.0,      384.6 / 383.0 / 384.1
+//   32^3 cavity, band 8 (1, 3)    66.1 /  68.0 /  68.0,       66.0 /  64.6 /  64.5
+//   band 16 (1, 4.7)              75.1 /  74.1 /  74.2,       72.1 /  71.6 /  72.0
+//   256x64x64 cylinder (2, 16.5) 160.7 / 156.2 / 156.1,      129.8 / 128.0 / 127.8
+//   refined less far (2, 13)     129.3 / 127.6 / 128.8,      117.9 / 116.7 / 117.5
+//   less still (2.6, 8)          100.9 / 103.2 /  98.8,      100.2 /  98.9 /  97.6
 // Over 28 such meshes: 0.992 of the time without (geometric mean) with the rule,
 // 0.994 with it always; single ones lie 1 - 3 % to either side.
 bool couple_triggers(const octlb_ctx* ctx, const Level& L) {
