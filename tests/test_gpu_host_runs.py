@@ -69,6 +69,38 @@ def test_interleaved_order_equals_level_order(ob, name, const_rho, prec):
         assert np.all(np.isfinite(a)) and np.array_equal(a[order], b)
 
 
+@pytest.mark.parametrize("const_rho", [False, True])
+def test_interleaved_order_with_fd_walls(ob, const_rho):
+    """The rewritten boundary cells' fields land in their blocks' places too."""
+    f = ob.Forest((1, 1, 1), (0, 0, 0), (0, 0, 0, 1, 1, 1)).refine_uniform(2)
+    f.refine_box((0.26, 0.26, 0.26, 0.74, 0.74, 0.74), 3).balance().build()
+    mesh = ob.Mesh.from_forest(f, 8)
+    types = [ob.FD_VELOCITY] * 6
+    u_wall = np.zeros((6, 3))
+    u_wall[3, 0] = 0.03
+    mesh = ob.stamp_fd_kinds(mesh, types)
+    sorted_mesh, order = by_level(ob, mesh)
+    assert not np.array_equal(order, np.arange(len(order)))
+    rng = np.random.default_rng(8)
+    shape = (mesh.n_blocks, 8, 8, 8)
+    rho, u = 1.0 + 0.01 * rng.standard_normal(shape), 0.02 * rng.standard_normal(shape + (3,))
+    res = []
+    for m, pick in ((mesh, np.arange(mesh.n_blocks)), (sorted_mesh, order)):
+        lat = ob.GpuLattice(m, 1.0 / 0.6)
+        if const_rho:
+            lat.set_const_rho(True)
+        lat.set_equilibrium(rho[pick].reshape(-1), u[pick].reshape(-1, 3))
+        lat.set_fd_boundary(types, u_wall)
+        out = []
+        for _ in range(2):
+            lat.advance(3)
+            out += [lat.get_populations(), *lat.get_fields()]
+        res.append([np.asarray(a).reshape((mesh.n_blocks, -1)) for a in out])
+        lat.close()
+    for a, b in zip(*res):
+        assert np.all(np.isfinite(a)) and np.array_equal(a[order], b)
+
+
 def test_staging_held_is_the_largest_level(ob):
     import torch
     from octlb_b200 import cases
